@@ -520,18 +520,6 @@ __device__ __forceinline__ fv::Cell<R> fv_cell(const R *stg, const R *uh, const 
     return c;
 }
 
-template <typename R>
-__device__ __forceinline__ fv::Grad<R> fv_grad(const fv::Cell<R> &lo, const fv::Cell<R> &c, const fv::Cell<R> &up, R theta)
-{
-    fv::Grad<R> g;
-    const R th = fv::theta_wd<R>(lo.dep, c.dep, up.dep, theta);
-    g.ds = fv::mc_half_gradient<R>(c.stg, lo.stg, up.stg, th);
-    g.dd = fv::mc_half_gradient<R>(c.dep, lo.dep, up.dep, th);
-    g.du = fv::mc_half_gradient<R>(c.u, lo.u, up.u, th);
-    g.dv = fv::mc_half_gradient<R>(c.v, lo.v, up.v, th);
-    return g;
-}
-
 // flux_NS(i, e+1, 1:3) (1-based edge e+1 = bottom edge of 0-based row e) or
 // flux_EW; zero where the reference never computes an edge.
 template <typename R, bool NS>
@@ -549,8 +537,8 @@ __device__ void fv_edge(const R *stg, const R *uh, const R *vh, const R *elv, in
             const int r = e0 - 2 + t;
             if (r >= 0 && r < ny) c[t] = fv_cell<R>(stg, uh, vh, elv, P, i0, r);
         }
-        gl = (e0 - 1 > 0 && e0 - 1 < ny - 1) ? fv_grad<R>(c[0], c[1], c[2], theta) : zero;
-        gh = (e0 > 0 && e0 < ny - 1) ? fv_grad<R>(c[1], c[2], c[3], theta) : zero;
+        gl = (e0 - 1 > 0 && e0 - 1 < ny - 1) ? fv::limited<R>(c[0], c[1], c[2], theta) : zero;
+        gh = (e0 > 0 && e0 < ny - 1) ? fv::limited<R>(c[1], c[2], c[3], theta) : zero;
         fv::EdgeRes<R> res;
         double cand;
         fv::edge_flux<R, true>(c[1], gl, c[2], gh, m.dxb[e0], R(1), res, cand, variant);
@@ -562,8 +550,8 @@ __device__ void fv_edge(const R *stg, const R *uh, const R *vh, const R *elv, in
             const int col = e0 - 2 + t;
             if (col >= 0 && col < nx) c[t] = fv_cell<R>(stg, uh, vh, elv, P, col, i0);
         }
-        gl = (e0 - 1 > 0 && e0 - 1 < nx - 1) ? fv_grad<R>(c[0], c[1], c[2], theta) : zero;
-        gh = (e0 > 0 && e0 < nx - 1) ? fv_grad<R>(c[1], c[2], c[3], theta) : zero;
+        gl = (e0 - 1 > 0 && e0 - 1 < nx - 1) ? fv::limited<R>(c[0], c[1], c[2], theta) : zero;
+        gh = (e0 > 0 && e0 < nx - 1) ? fv::limited<R>(c[1], c[2], c[3], theta) : zero;
         fv::EdgeRes<R> res;
         double cand;
         fv::edge_flux<R, false>(c[1], gl, c[2], gh, m.dyl[e0], R(1), res, cand, variant);

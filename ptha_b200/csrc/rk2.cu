@@ -141,11 +141,7 @@ __global__ void __launch_bounds__(NT, 3) rk2_stage_kernel(const Rk2Args<R> a)
         Grad<R> g; g.ds = R(0); g.dd = R(0); g.du = R(0); g.dv = R(0);
         if (r > 0 && r < ny - 1 && i < nx) {
             const Cell<R> lo = S.cell.get(rr, cc + 2), c = S.cell.get(rr + 1, cc + 2), up = S.cell.get(rr + 2, cc + 2);
-            const R th = theta_wd<R>(lo.dep, c.dep, up.dep, a.theta);
-            g.ds = mc_half_gradient<R>(c.stg, lo.stg, up.stg, th);
-            g.dd = mc_half_gradient<R>(c.dep, lo.dep, up.dep, th);
-            g.du = mc_half_gradient<R>(c.u, lo.u, up.u, th);
-            g.dv = mc_half_gradient<R>(c.v, lo.v, up.v, th);
+            g = limited<R>(lo, c, up, a.theta);
         }
         S.gns.set(rr, cc, g);
     }
@@ -155,11 +151,7 @@ __global__ void __launch_bounds__(NT, 3) rk2_stage_kernel(const Rk2Args<R> a)
         Grad<R> g; g.ds = R(0); g.dd = R(0); g.du = R(0); g.dv = R(0);
         if (i > 0 && i < nx - 1 && r < ny) {
             const Cell<R> lo = S.cell.get(rr + 2, cc), c = S.cell.get(rr + 2, cc + 1), up = S.cell.get(rr + 2, cc + 2);
-            const R th = theta_wd<R>(lo.dep, c.dep, up.dep, a.theta);
-            g.ds = mc_half_gradient<R>(c.stg, lo.stg, up.stg, th);
-            g.dd = mc_half_gradient<R>(c.dep, lo.dep, up.dep, th);
-            g.du = mc_half_gradient<R>(c.u, lo.u, up.u, th);
-            g.dv = mc_half_gradient<R>(c.v, lo.v, up.v, th);
+            g = limited<R>(lo, c, up, a.theta);
         }
         S.gew.set(rr, cc, g);
     }
@@ -179,7 +171,7 @@ __global__ void __launch_bounds__(NT, 3) rk2_stage_kernel(const Rk2Args<R> a)
                                      S.gns.get(rr + 1, cc), a.m.dxb[r], inv2, e, cand, a.flux_variant,
                                      EDDY ? a.ev[(int64_t)(r - 1) * a.P + i] : R(0),
                                      EDDY ? a.ev[(int64_t)r * a.P + i] : R(0), EDDY ? a.m.dyl[i] : R(1));
-            cfl = fmax(cfl, cand);
+            cfl = rmax(cfl, cand);
             if (MODE != MODE_CFL && a.lines) {
                 if (r == ny - a.n_ext && i >= a.n_ext && i <= nx - a.n_ext - 1) a.lines[i] = (double)e.f[0];
                 if (r == a.n_ext && i >= a.n_ext && i <= nx - a.n_ext - 1) a.lines[nx + ny + i] = (double)e.f[0];
@@ -200,7 +192,7 @@ __global__ void __launch_bounds__(NT, 3) rk2_stage_kernel(const Rk2Args<R> a)
                                       S.gew.get(rr, cc + 1), a.m.dyl[i], inv1, e, cand, a.flux_variant,
                                       EDDY ? a.ev[oe - 1] : R(0), EDDY ? a.ev[oe] : R(0),
                                       EDDY ? R(0.5) * (a.m.dxb[r] + a.m.dxb[r + 1]) : R(1));
-            cfl = fmax(cfl, cand);
+            cfl = rmax(cfl, cand);
             if (MODE != MODE_CFL && a.lines) {
                 if (i == nx - a.n_ext && r >= a.n_ext && r <= ny - a.n_ext - 1) a.lines[nx + r] = (double)e.f[0];
                 if (i == a.n_ext && r >= a.n_ext && r <= ny - a.n_ext - 1) a.lines[2 * nx + ny + r] = (double)e.f[0];
@@ -636,7 +628,7 @@ __device__ __forceinline__ void update_cell(const Rk2Args<R> &a, int i, int r, R
     R dep = sv - ev;
     c.u = R(0); c.v = R(0);
     if (dep > K<R>::min_depth()) {
-        const R depth_inv = R(1) / dep;
+        const R depth_inv = depth_inverse(dep);
         c.u = uh_in * depth_inv;
         c.v = vh_in * depth_inv;
     } else if (dep < R(0)) {
@@ -764,7 +756,7 @@ __global__ void __launch_bounds__(256) eddy_visc_kernel(const Rk2Args<R> a)
     const int64_t o = (int64_t)r * a.P + is;
     R dep = a.stg[o] - a.elv[o], u = R(0), v = R(0);
     if (dep > K<R>::min_depth()) {
-        const R depth_inv = R(1) / dep;
+        const R depth_inv = depth_inverse(dep);
         u = a.uh[o] * depth_inv;
         v = a.vh[o] * depth_inv;
     } else if (dep < R(0)) {

@@ -87,7 +87,7 @@ __device__ __forceinline__ Cell<R> fix_up(const Raw<R> &x, bool valid, long long
         const R e = x.e;
         R dep = s - e;
         if (dep > K<R>::min_depth()) {
-            const R depth_inv = R(1) / dep;
+            const R depth_inv = depth_inverse(dep);
             c.u = x.uh * depth_inv;
             c.v = x.vh * depth_inv;
         } else if (dep < R(0)) {
@@ -115,18 +115,6 @@ template <typename R>
 __device__ __forceinline__ Cell<R> dn1(const Cell<R> &c)
 {
     Cell<R> x; x.stg = dn1(c.stg); x.dep = dn1(c.dep); x.u = dn1(c.u); x.v = dn1(c.v); x.elv = dn1(c.elv); return x;
-}
-
-template <typename R>
-__device__ __forceinline__ Grad<R> limited(const Cell<R> &lo, const Cell<R> &c, const Cell<R> &up, R theta)
-{
-    Grad<R> g;
-    const R th = theta_wd<R>(lo.dep, c.dep, up.dep, theta);
-    g.ds = mc_half_gradient<R>(c.stg, lo.stg, up.stg, th);
-    g.dd = mc_half_gradient<R>(c.dep, lo.dep, up.dep, th);
-    g.du = mc_half_gradient<R>(c.u, lo.u, up.u, th);
-    g.dv = mc_half_gradient<R>(c.v, lo.v, up.v, th);
-    return g;
 }
 
 template <typename R>
@@ -222,7 +210,7 @@ __global__ void __launch_bounds__(SLANES *SWARPS, SWALS_STREAM_MIN_CTAS) rk2_str
                 edge_flux<R, true, EDDY>(c2, g2, c1, g1, a.m.dxb[e], inv2, e_n, cand, a.flux_variant,
                                          EDDY ? a.ev[(int64_t)(e - 1) * a.P + i] : R(0),
                                          EDDY ? a.ev[(int64_t)e * a.P + i] : R(0), EDDY ? a.m.dyl[i] : R(1));
-                if (MODE != MODE_STAGE2) cfl = fmax(cfl, cand);   // stage 2 writes no CFL
+                if (MODE != MODE_STAGE2) cfl = rmax(cfl, cand);   // stage 2 writes no CFL
                 if (MODE != MODE_CFL && a.lines && i >= a.n_ext && i <= nx - a.n_ext - 1) {
                     if (e == ny - a.n_ext) a.lines[i] = (double)e_n.f[0];
                     if (e == a.n_ext) a.lines[nx + ny + i] = (double)e_n.f[0];
@@ -248,7 +236,7 @@ __global__ void __launch_bounds__(SLANES *SWARPS, SWALS_STREAM_MIN_CTAS) rk2_str
             edge_flux<R, false, EDDY>(cl, gw, c2, gew, a.m.dyl[i], inv1, e_w, cand, a.flux_variant,
                                       EDDY ? a.ev[oe - 1] : R(0), EDDY ? a.ev[oe] : R(0),
                                       EDDY ? R(0.5) * (a.m.dxb[R_] + a.m.dxb[R_ + 1]) : R(1));
-            if (MODE != MODE_STAGE2) cfl = fmax(cfl, cand);
+            if (MODE != MODE_STAGE2) cfl = rmax(cfl, cand);
             if (MODE != MODE_CFL && a.lines && R_ >= a.n_ext && R_ <= ny - a.n_ext - 1) {
                 if (i == nx - a.n_ext) a.lines[nx + R_] = (double)e_w.f[0];
                 if (i == a.n_ext) a.lines[2 * nx + ny + R_] = (double)e_w.f[0];
@@ -421,7 +409,7 @@ __global__ void __launch_bounds__(SLANES *SWARPS, srow_min_ctas(MODE, SW, EDDY, 
                                          a.m.dxb[e], inv2, e_n, cand, a.flux_variant,
                                          EDDY ? a.ev[(int64_t)(e - 1) * a.P + i] : R(0),
                                          EDDY ? a.ev[(int64_t)e * a.P + i] : R(0), EDDY ? a.m.dyl[i] : R(1));
-                if (MODE != MODE_STAGE2) cfl = fmax(cfl, cand);   // stage 2 writes no CFL
+                if (MODE != MODE_STAGE2) cfl = rmax(cfl, cand);   // stage 2 writes no CFL
                 // the boundary-flux lines (rows n_ext and ny - n_ext): tested
                 // on the row first, the same for the whole strip
                 if (MODE != MODE_CFL && (e == ny - a.n_ext || e == a.n_ext) && a.lines && i >= a.n_ext &&
@@ -447,7 +435,7 @@ __global__ void __launch_bounds__(SLANES *SWARPS, srow_min_ctas(MODE, SW, EDDY, 
             edge_flux<R, false, EDDY>(sm.c[s2][lw], gw[lw], sm.c[s2][lane], gw[lane], a.m.dyl[i], inv1, e_w,
                                       cand, a.flux_variant, EDDY ? a.ev[oe - 1] : R(0), EDDY ? a.ev[oe] : R(0),
                                       EDDY ? R(0.5) * (a.m.dxb[R_] + a.m.dxb[R_ + 1]) : R(1));
-            if (MODE != MODE_STAGE2) cfl = fmax(cfl, cand);
+            if (MODE != MODE_STAGE2) cfl = rmax(cfl, cand);
             if (MODE != MODE_CFL && (i == nx - a.n_ext || i == a.n_ext) && a.lines && R_ >= a.n_ext &&
                 R_ <= ny - a.n_ext - 1) {
                 if (i == nx - a.n_ext) a.lines[nx + R_] = (double)e_w.f[0];

@@ -34,6 +34,63 @@ template <typename R> struct K {
 template <typename R> __device__ __forceinline__ R rmin(R a, R b) { return (b < a) ? b : a; }
 template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return (b > a) ? b : a; }
 
+// Correctly rounded FP64 reciprocal, quotient and square root for operands of
+// ordinary size, without a branch: Newton's iteration from the hardware's
+// approximations (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64), then
+// Markstein's final correction from the exact remainder (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34, 1990).  The compiler's own sequences test
+// their operands' range and branch to a general routine; between those
+// branches the scheduler cannot interleave the independent square roots and
+// quotients of an edge, and the stage kernels are bound by exactly that
+// latency.  Here the callers see to the range and use the plain operators
+// outside it: operands, results and remainders between 1e-290 and 1e290, so
+// that nothing overflows, underflows or is infinite.  sqrt_ord takes what is
+// below 1e-290, zero included, as zero.  Compared with the correctly rounded
+// instructions on 2.5e10 operands of each, a quarter of them with
+// significands near 1 or 2: no difference.
+// 1/b within about an ulp.
+__device__ __forceinline__ double rcp_near(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = fma(-b, y, 1.0);
+    e = fma(e, e, e);
+    return fma(y, e, y);
+}
+// Markstein's one exception, a significand of b of all ones: 1/b lies just
+// above the middle of 2^k and its successor, and rounds to the latter.
+__device__ __forceinline__ double rcp_of_ones(double b, double y)
+{
+    const int lo = __double2loint(b), hi = __double2hiint(b);
+    const bool ones = (lo & (hi | ~0xfffff)) == -1;
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
+}
+__device__ __forceinline__ double rcp_ord(double b)
+{
+    const double y = rcp_near(b);
+    return rcp_of_ones(b, fma(y, fma(-b, y, 1.0), y));
+}
+__device__ __forceinline__ float rcp_ord(float b) { return 1.0f / b; }
+__device__ __forceinline__ double div_ord(double a, double b)
+{
+    const double y = rcp_of_ones(b, rcp_near(b));
+    double q = a * y;
+    q = fma(fma(-b, q, a), y, q);          // within half an ulp and a little
+    return fma(fma(-b, q, a), y, q);       // from its exact remainder
+}
+__device__ __forceinline__ double sqrt_ord(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    y = fma(fma(0.375, e, 0.5), y * e, y);
+    const double g = x * y;
+    const double r = fma(fma(-g, g, x), 0.5 * y, g);
+    return (x < 1.0e-290) ? 0.0 : r;
+}
+__device__ __forceinline__ float sqrt_ord(float x) { return sqrtf(x); }
+
 // Friction power law pow(x, p), p = fl(-7/3) (Manning) or -2 (Chezy), for
 // x >= minimum_allowed_depth (update_U_DE1_inner_include.f90:72-75).  The
 // oracle evaluates the same operation sequence, so both give the same bits
@@ -65,7 +122,8 @@ __device__ __forceinline__ DD dd_recip(DD p)
 }
 constexpr unsigned kRcbrtSeed = 0x54a237fbu;
 constexpr double kEpsLn2 = -1.0260639457488826e-16;   // (fl(-7/3) + 7/3) ln 2
-template <bool CHEZY>
+// ORD: x is of ordinary size (up to 1e30, in range for the FP32 seed).
+template <bool CHEZY, bool ORD = false>
 __device__ __forceinline__ double pow_friction(double x)
 {
     if (CHEZY) return dd_recip(dd_two_prod(x, x)).hi;
@@ -78,7 +136,7 @@ __device__ __forceinline__ double pow_friction(double x)
     double yd = (double)y;
     yd = yd + yd * ((1.0 - x * (yd * yd * yd)) * (1.0 / 3.0));
     yd = yd + yd * ((1.0 - x * (yd * yd * yd)) * (1.0 / 3.0));
-    const double v = yd / (x * x);
+    const double v = ORD ? div_ord(yd, x * x) : yd / (x * x);
     const double t = kEpsLn2 * ((double)ix * (1.0 / 8388608.0) - 127.0);
     return v + v * t;
 }
