@@ -640,7 +640,9 @@ __device__ __forceinline__ void update_cell(const Rk2Args<R> &a, int i, int r, R
     // U(i,j,UH/VH) after the fix-ups (fixed_momenta)
     const bool wet = c.dep > K<R>::min_depth();
     const R Um_uh = wet ? uh_in : R(0), Um_vh = wet ? vh_in : R(0);
-    fv_apply<R, MODE_STAGE1, FRIC>(a, i, r, c, Um_uh, Um_vh, f, dt, dt / area);
+    fv_apply<R, MODE_STAGE1>(a, i, r, c, Um_uh, Um_vh, f, dt / area,
+                             [&] { return friction_factor<R, FRIC>(a, FRIC == FRIC_NONE ? R(0) : a.nsq[(int64_t)r * a.P + i], c, dt); },
+                             Stage2Mem<R>());
 }
 
 // Cells per thread and CTAs per SM of the stage-1 update.  Measured on the

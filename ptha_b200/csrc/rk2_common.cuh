@@ -168,6 +168,30 @@ __device__ __forceinline__ Grad<R> limited(const Cell<R> &cl, const Cell<R> &c, 
     return g;
 }
 
+// Stage, depth and velocities reconstructed at an edge of a cell
+// (DE1_inner_include.f90's U +- 1/2 gradient; Grad holds twice the gradient).
+template <typename R> struct Face { R s, d, u, v; };
+template <typename R>
+__device__ __forceinline__ Face<R> face_above(const Cell<R> &c, const Grad<R> &g)   // the north or east edge
+{
+    const R q = R(0.25);
+    Face<R> f;
+    f.s = fma(q, g.ds, c.stg); f.d = fma(q, g.dd, c.dep); f.u = fma(q, g.du, c.u); f.v = fma(q, g.dv, c.v);
+    return f;
+}
+template <typename R>
+__device__ __forceinline__ Face<R> face_below(const Cell<R> &c, const Grad<R> &g)   // the south or west edge
+{
+    const R q = R(-0.25);
+    Face<R> f;
+    f.s = fma(q, g.ds, c.stg); f.d = fma(q, g.dd, c.dep); f.u = fma(q, g.du, c.u); f.v = fma(q, g.dv, c.v);
+    return f;
+}
+
+// What the *_eddyvisc variants add to an edge: the eddy viscosities of the two
+// cells, the velocity differences and the distance they are taken over.
+template <typename R> struct EddyIn { R ev_n, ev_p, du, dv, vel_div; };
+
 template <typename R>
 struct EdgeRes {
     R f[3];          // STG, UH, VH flux (already multiplied by edge length)
@@ -197,14 +221,14 @@ __device__ __forceinline__ R eddy_momentum_flux(R adv, R hll, R turb)
 // 0.071; midpoint on a spherical 930^2 patch 0.196 -> 0.167.
 // NS=true: normal velocity v, edge between (i,j-1) and (i,j).
 // variant: compute_fluxes_inner_method as FLUX_* bits (swals_kernels.h);
-// 0 is the default 'DE1_low_fr_diffusion'.  EDDY (FLUX_EDDY): ev_n / ev_p are
-// the eddy viscosities of the two cells and vel_div the distance the
-// velocity difference is taken over (distance_left_edge(i) for NS edges,
-// the mean of distance_bottom_edge(j), (j+1) for EW edges).
+// 0 is the default 'DE1_low_fr_diffusion'.  EDDY (FLUX_EDDY): vel_div is
+// distance_left_edge(i) for NS edges, the mean of distance_bottom_edge(j),
+// (j+1) for EW edges.  n, p: the faces of the two cells at the edge, dep_ and
+// elv_ their depths and elevations.
 template <typename R, bool NS, bool EDDY = false>
-__device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, const Cell<R> &cp, const Grad<R> &gp,
-                                          R edge_len, R dx_cfl_half_inv, EdgeRes<R> &out, double &cfl_cand,
-                                          int variant = 0, R ev_n = R(0), R ev_p = R(0), R vel_div = R(1))
+__device__ __forceinline__ void edge_faces(const Face<R> &n, R dep_n, R elv_n, const Face<R> &p, R dep_p, R elv_p,
+                                           R edge_len, EdgeRes<R> &out, R &max_speed, int variant = 0,
+                                           const EddyIn<R> &eddy = EddyIn<R>())
 {
     const R half = R(0.5);
     const double half_gravity = (double)(half * K<R>::gravity());
@@ -213,48 +237,37 @@ __device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, 
     // correctly rounded root of the rounded product, as written out here)
     const R EPS_gs = sizeof(R) == 8 ? R(0x1.4462fb7ff5035p-7) : R(0x1.4462fcp-7f);
     const R beta = R(1.0);
-
-    // (gn, gp hold twice the gradients: DE1_inner_include.f90's U +- 1/2 grad)
-    const R quarter = R(0.25);
-    const R stage_neg = fma(quarter, gn.ds, cn.stg);
-    const R stage_pos = fma(-quarter, gp.ds, cp.stg);
-    const double depth_neg = (double)fma(quarter, gn.dd, cn.dep);
-    const double depth_pos = (double)fma(-quarter, gp.dd, cp.dep);
-    R u_neg = fma(quarter, gn.du, cn.u);
-    R u_pos = fma(-quarter, gp.du, cp.u);
-    R v_neg = fma(quarter, gn.dv, cn.v);
-    R v_pos = fma(-quarter, gp.dv, cp.v);
-    const double depth_neg_c = (double)cn.dep;
-    const double depth_pos_c = (double)cp.dep;
-
-    const R z_neg = R((double)stage_neg - depth_neg);
-    const R z_pos = R((double)stage_pos - depth_pos);
+    // (Sums, differences and products that the reference forms in double from
+    // two values of the state precision and rounds to it are formed in the
+    // state precision here: with 53 bits against 24 the second rounding
+    // changes nothing.)
+    const R z_neg = n.s - n.d;
+    const R z_pos = p.s - p.d;
     const R z_half = rmax(z_neg, z_pos);
 
     // a side's depth at the edge is zero exactly where its stage is not above z_half
-    const bool dry_neg = z_half >= stage_neg, dry_pos = z_half >= stage_pos;
-    const R stage_neg_star = dry_neg ? z_half : stage_neg;
-    const R stage_pos_star = dry_pos ? z_half : stage_pos;
-    const double depth_neg_star = (double)(stage_neg_star - z_half);
-    const double depth_pos_star = (double)(stage_pos_star - z_half);
-    if (dry_neg) { u_neg = R(0); v_neg = R(0); }
-    if (dry_pos) { u_pos = R(0); v_pos = R(0); }
-    const R ud_neg = R((double)u_neg * depth_neg_star);
-    const R vd_neg = R((double)v_neg * depth_neg_star);
-    R gs_neg = R(sqrt_ord((double)K<R>::gravity() * depth_neg_star));
-    const R ud_pos = R((double)u_pos * depth_pos_star);
-    const R vd_pos = R((double)v_pos * depth_pos_star);
-    R gs_pos = R(sqrt_ord((double)K<R>::gravity() * depth_pos_star));
-
+    const bool dry_neg = z_half >= n.s, dry_pos = z_half >= p.s;
+    const R stage_neg_star = dry_neg ? z_half : n.s;
+    const R stage_pos_star = dry_pos ? z_half : p.s;
+    const R d_neg = stage_neg_star - z_half, d_pos = stage_pos_star - z_half;
+    const double depth_neg = (double)n.d, depth_pos = (double)p.d;
+    const double depth_neg_star = (double)d_neg, depth_pos_star = (double)d_pos;
+    const R u_neg = dry_neg ? R(0) : n.u, v_neg = dry_neg ? R(0) : n.v;
+    const R u_pos = dry_pos ? R(0) : p.u, v_pos = dry_pos ? R(0) : p.v;
     const R vel_beta_neg = (NS ? v_neg : u_neg) * beta;
     const R vel_beta_pos = (NS ? v_pos : u_pos) * beta;
+    const R tran_neg = NS ? u_neg : v_neg, tran_pos = NS ? u_pos : v_pos;
+    const R qn_neg = vel_beta_neg * d_neg, qn_pos = vel_beta_pos * d_pos;
+    const R qt_neg = tran_neg * d_neg, qt_pos = tran_pos * d_pos;
+    R gs_neg = R(sqrt_ord((double)K<R>::gravity() * depth_neg_star));
+    R gs_pos = R(sqrt_ord((double)K<R>::gravity() * depth_pos_star));
 
     R s_max = rmax(rmax(vel_beta_neg + gs_neg, vel_beta_pos + gs_pos), R(0));
     R s_min = rmin(rmin(vel_beta_neg - gs_neg, vel_beta_pos - gs_pos), R(0));
     double denom = (double)(s_max - s_min);
     double quotient = div_ord((double)edge_len, denom);   // unused where denom is tiny
-    const double depth_sum = depth_neg_star + depth_pos_star;
-    if (!(depth_sum < 1.0e280 && denom < 1.0e280)) {   // a run that has blown up: the plain operators
+    const R depth_sum = d_neg + d_pos;
+    if (!((double)depth_sum < 1.0e280 && denom < 1.0e280)) {   // a run that has blown up: the plain operators
         gs_neg = R(sqrt((double)K<R>::gravity() * depth_neg_star));
         gs_pos = R(sqrt((double)K<R>::gravity() * depth_pos_star));
         s_max = rmax(rmax(vel_beta_neg + gs_neg, vel_beta_pos + gs_pos), R(0));
@@ -271,8 +284,9 @@ __device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, 
     // edges form it.
     R fr2 = R(1);
     if (!(variant & FLUX_PLAIN_DIFFUSION)) {
-        const R num_b = fma(v_neg, v_neg, fma(v_pos, v_pos, fma(u_neg, u_neg, u_pos * u_pos)));
-        const R den_b = K<R>::gravity() * R(depth_sum) + R(1.0e-10);
+        const R num_b = fma(vel_beta_neg, vel_beta_neg,
+                            fma(vel_beta_pos, vel_beta_pos, fma(tran_neg, tran_neg, tran_pos * tran_pos)));
+        const R den_b = K<R>::gravity() * depth_sum + R(1.0e-10);
         fr2 = sizeof(R) == 8 ? R(0x1.030dc4ea03a72p-5) : R(0x1.030dc6p-5f);
         if (!(num_b < R(0.00099) * den_b)) {
             const R fr2num = ((v_neg * v_neg + v_pos * v_pos) + u_neg * u_neg) + u_pos * u_pos;
@@ -282,8 +296,6 @@ __device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, 
         fr2 = beta * fr2;
     }
 
-    const R qn_neg = NS ? vd_neg : ud_neg, qn_pos = NS ? vd_pos : ud_pos;
-    const R qt_neg = NS ? ud_neg : vd_neg, qt_pos = NS ? ud_pos : vd_pos;
     const R f_mass = R((double)((s_max * qn_neg - s_min * qn_pos) + sminsmax * (stage_pos_star - stage_neg_star)) *
                        inv_denom);
     R f_norm, f_tran;
@@ -291,27 +303,27 @@ __device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, 
         f_norm = R((double)((s_max * qn_neg * vel_beta_neg - s_min * qn_pos * vel_beta_pos) +
                             fr2 * sminsmax * (qn_pos - qn_neg)) * inv_denom);
         if (variant & FLUX_UPWIND_TRANSVERSE)   // upwind_transverse_momentum: the transverse velocity upwind of the mass flux
-            f_tran = beta * ((f_mass > R(0)) ? (NS ? u_neg : v_neg) : (NS ? u_pos : v_pos)) * f_mass;
+            f_tran = beta * ((f_mass > R(0)) ? tran_neg : tran_pos) * f_mass;
         else
             f_tran = R((double)((s_max * qt_neg * vel_beta_neg - s_min * qt_pos * vel_beta_pos) +
                                 fr2 * sminsmax * (qt_pos - qt_neg)) * inv_denom);
     } else {
         // turbulent diffusion: eddy_visc * depth * edge length * velocity gradient,
         // with the geometric mean of the edge depths
-        const R evh = half * (ev_p + ev_n);
+        const R evh = half * (eddy.ev_p + eddy.ev_n);
         const R gdep = R(sqrt(depth_neg_star * depth_pos_star));
         R adv = R((double)(s_max * qn_neg * vel_beta_neg - s_min * qn_pos * vel_beta_pos) * inv_denom);
         R hll = R((double)(fr2 * sminsmax * (qn_pos - qn_neg)) * inv_denom);
-        R turb = -(evh * gdep * edge_len * ((NS ? (cp.v - cn.v) : (cp.u - cn.u)) / vel_div));
+        R turb = -(evh * gdep * edge_len * ((NS ? eddy.dv : eddy.du) / eddy.vel_div));
         f_norm = eddy_momentum_flux<R>(adv, hll, turb);
         if (variant & FLUX_UPWIND_TRANSVERSE) {
-            adv = beta * ((f_mass > R(0)) ? (NS ? u_neg : v_neg) : (NS ? u_pos : v_pos)) * f_mass;
+            adv = beta * ((f_mass > R(0)) ? tran_neg : tran_pos) * f_mass;
             hll = R(0);
         } else {
             adv = R((double)(s_max * qt_neg * vel_beta_neg - s_min * qt_pos * vel_beta_pos) * inv_denom);
             hll = R((double)(fr2 * sminsmax * (qt_pos - qt_neg)) * inv_denom);
         }
-        turb = -(evh * gdep * edge_len * ((NS ? (cp.u - cn.u) : (cp.v - cn.v)) / vel_div));
+        turb = -(evh * gdep * edge_len * ((NS ? eddy.du : eddy.dv) / eddy.vel_div));
         f_tran = eddy_momentum_flux<R>(adv, hll, turb);
     }
     out.f[0] = f_mass;
@@ -321,17 +333,35 @@ __device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, 
     const double half_g_hh_edge = inv_denom * half_gravity *
         ((double)s_max * depth_neg_star * depth_neg_star - (double)s_min * depth_pos_star * depth_pos_star);
     const double bs_neg = half_gravity * ((depth_neg_star - depth_neg) * (depth_neg_star + depth_neg) -
-                                          (depth_neg + depth_neg_c) * (double)(z_neg - cn.elv));
+                                          (depth_neg + (double)dep_n) * (double)(z_neg - elv_n));
     out.es_neg = bs_neg * (double)edge_len - half_g_hh_edge;
     const double bs_pos = half_gravity * ((depth_pos_star - depth_pos) * (depth_pos_star + depth_pos) -
-                                          (depth_pos + depth_pos_c) * (double)(z_pos - cp.elv));
+                                          (depth_pos + (double)dep_p) * (double)(z_pos - elv_p));
     out.es_pos = half_g_hh_edge - bs_pos * (double)edge_len;
 
-    const double max_speed = (double)rmax(s_max, -s_min);
-    cfl_cand = (max_speed > (double)EPS) ? max_speed * (double)dx_cfl_half_inv : 0.0;
+    max_speed = rmax(s_max, -s_min);
 }
 
+// A speed's candidate for the largest 1/dt of its edge.
+template <typename R>
+__device__ __forceinline__ double cfl_rate(R max_speed, R dx_cfl_half_inv)
+{
+    return (max_speed > R(1.0e-12)) ? (double)max_speed * (double)dx_cfl_half_inv : 0.0;
+}
 
+// The edge between two cells from their values and (twice the) gradients.
+template <typename R, bool NS, bool EDDY = false>
+__device__ __forceinline__ void edge_flux(const Cell<R> &cn, const Grad<R> &gn, const Cell<R> &cp, const Grad<R> &gp,
+                                          R edge_len, R dx_cfl_half_inv, EdgeRes<R> &out, double &cfl_cand,
+                                          int variant = 0, R ev_n = R(0), R ev_p = R(0), R vel_div = R(1))
+{
+    EddyIn<R> eddy;
+    if (EDDY) { eddy.ev_n = ev_n; eddy.ev_p = ev_p; eddy.vel_div = vel_div; eddy.du = cp.u - cn.u; eddy.dv = cp.v - cn.v; }
+    R max_speed;
+    edge_faces<R, NS, EDDY>(face_above(cn, gn), cn.dep, cn.elv, face_below(cp, gp), cp.dep, cp.elv, edge_len, out,
+                            max_speed, variant, eddy);
+    cfl_cand = cfl_rate<R>(max_speed, dx_cfl_half_inv);
+}
 
 // Timestep of a stage: fixed, or domain%max_dt of the first stage
 // 1/max(1/maximum_timestep, max speed/(dx cfl/2)) for adaptive stepping.
@@ -402,14 +432,50 @@ __device__ __forceinline__ void fixed_momenta(const Rk2Args<R> &a, int64_t o, co
     else { Um_uh = R(0); Um_vh = R(0); }
 }
 
+// The semi-implicit friction factor of cell o of the stage input (1 without friction).
+template <typename R, int FRIC>
+__device__ __forceinline__ R friction_factor(const Rk2Args<R> &a, R nsq, const Cell<R> &c, R dt)
+{
+    if (FRIC == FRIC_NONE) return R(1);
+    constexpr bool CHEZY = (FRIC == FRIC_CHEZY);
+    const R mad = K<R>::min_depth();
+    const R depth = c.dep;
+    const R speed2 = c.u * c.u + c.v * c.v;
+    const R dg = dt * K<R>::gravity() * rmax(depth, R(0));
+    if ((double)depth < 1.0e30 && (double)speed2 < 1.0e280) {
+        const R fs = nsq * sqrt_ord(speed2) * R(pow_friction<CHEZY, true>((double)rmax(depth, mad)));
+        return rcp_ord((R(1) + dg * fs) + dt * a.lin_fric);
+    }
+    // a run that has blown up: the plain operators
+    const R fs = nsq * R(sqrt(speed2)) * R(pow_friction<CHEZY>((double)rmax(depth, mad)));
+    return R(1) / ((R(1) + dg * fs) + dt * a.lin_fric);
+}
+
+// Stage 2's U0 and max_stage of a cell: read where they are used, or loaded
+// ahead by the caller.
+template <typename R> struct Stage2Mem {
+    __device__ __forceinline__ R s(const Rk2Args<R> &a, int64_t o) const { return a.stg0[o]; }
+    __device__ __forceinline__ R uh(const Rk2Args<R> &a, int64_t o) const { return a.uh0[o]; }
+    __device__ __forceinline__ R vh(const Rk2Args<R> &a, int64_t o) const { return a.vh0[o]; }
+    __device__ __forceinline__ R mx(const Rk2Args<R> &a, int64_t o) const { return a.max_stage[o]; }
+};
+template <typename R> struct Stage2Reg {
+    R s_, uh_, vh_, mx_;
+    __device__ __forceinline__ R s(const Rk2Args<R> &, int64_t) const { return s_; }
+    __device__ __forceinline__ R uh(const Rk2Args<R> &, int64_t) const { return uh_; }
+    __device__ __forceinline__ R vh(const Rk2Args<R> &, int64_t) const { return vh_; }
+    __device__ __forceinline__ R mx(const Rk2Args<R> &, int64_t) const { return mx_; }
+};
+
 // The rest of update_U for cell (i, r) with the stage's dt: the flux
 // update, the wet/dry test, the semi-implicit friction and the explicit
 // sources; stage 2 also forms the rk2 average and max_stage.
 // inv_cell_area_dt is the row's dt / area_cell_y(r) (a row constant the
-// callers may evaluate once per row).
-template <typename R, int MODE, int FRIC>
+// callers may evaluate once per row); factor() gives the friction factor, in
+// gives stage 2's U0 and max_stage of the cell (Stage2Mem, Stage2Reg).
+template <typename R, int MODE, typename Factor, typename Stage2>
 __device__ __forceinline__ void fv_apply(const Rk2Args<R> &a, int i, int r, const Cell<R> &c, R Um_uh, R Um_vh,
-                                         const CellFlux<R> &f, R dt, R inv_cell_area_dt)
+                                         const CellFlux<R> &f, R inv_cell_area_dt, Factor factor, Stage2 in)
 {
     const int nx = a.nx, ny = a.ny;
     const int64_t P = a.P;
@@ -431,22 +497,7 @@ __device__ __forceinline__ void fv_apply(const Rk2Args<R> &a, int i, int r, cons
         U_uh = R(0);
         U_vh = R(0);
     } else {
-        R implicit_factor;
-        if (FRIC == FRIC_NONE) {
-            implicit_factor = R(1);
-        } else {
-            const R depth = c.dep;
-            const R speed2 = c.u * c.u + c.v * c.v;
-            const R dg = dt * K<R>::gravity() * rmax(depth, R(0));
-            constexpr bool CHEZY = (FRIC == FRIC_CHEZY);
-            if ((double)depth < 1.0e30 && (double)speed2 < 1.0e280) {
-                const R fs = a.nsq[o] * sqrt_ord(speed2) * R(pow_friction<CHEZY, true>((double)rmax(depth, mad)));
-                implicit_factor = rcp_ord((R(1) + dg * fs) + dt * a.lin_fric);
-            } else {   // a run that has blown up: the plain operators
-                const R fs = a.nsq[o] * R(sqrt(speed2)) * R(pow_friction<CHEZY>((double)rmax(depth, mad)));
-                implicit_factor = R(1) / ((R(1) + dg * fs) + dt * a.lin_fric);
-            }
-        }
+        const R implicit_factor = factor();
         U_uh = R((double)U_uh + (double)inv_cell_area_dt * f.eu);
         U_uh = U_uh * implicit_factor;
         U_vh = R((double)U_vh + (double)inv_cell_area_dt * f.ev);
@@ -471,14 +522,14 @@ __device__ __forceinline__ void fv_apply(const Rk2Args<R> &a, int i, int r, cons
                 }
             }
         }
-        U_stg = R(0.5) * (U_stg + a.stg0[o]);
-        U_uh = R(0.5) * (U_uh + a.uh0[o]);
-        U_vh = R(0.5) * (U_vh + a.vh0[o]);
+        U_stg = R(0.5) * (U_stg + in.s(a, o));
+        U_uh = R(0.5) * (U_uh + in.uh(a, o));
+        U_vh = R(0.5) * (U_vh + in.vh(a, o));
         if (a.max_stage) {
             const bool ring = a.bc_ring && outer2 && ((i == 0 && a.bext[3]) || (i == nx - 1 && a.bext[1]) ||
                                                       (r == 0 && a.bext[2]) || (r == ny - 1 && a.bext[0]));
             if (!ring) {
-                R mx = a.max_stage[o];
+                R mx = in.mx(a, o);
                 a.max_stage[o] = (U_stg > mx) ? U_stg : mx;
             }
         }
@@ -498,7 +549,9 @@ __device__ __forceinline__ void fv_update(const Rk2Args<R> &a, int i, int r, con
     R Um_uh, Um_vh;
     fixed_momenta<R>(a, (int64_t)r * a.P + i, c, Um_uh, Um_vh);
     const CellFlux<R> f = cell_flux<R, SPH, COR>(a, i, r, c, Um_uh, Um_vh, n_lo, n_hi, w_lo, w_hi);
-    fv_apply<R, MODE, FRIC>(a, i, r, c, Um_uh, Um_vh, f, dt, inv_cell_area_dt);
+    fv_apply<R, MODE>(a, i, r, c, Um_uh, Um_vh, f, inv_cell_area_dt,
+                      [&] { return friction_factor<R, FRIC>(a, FRIC == FRIC_NONE ? R(0) : a.nsq[(int64_t)r * a.P + i], c, dt); },
+                      Stage2Mem<R>());
 }
 }  // namespace fv
 }  // namespace swals
