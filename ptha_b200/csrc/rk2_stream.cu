@@ -281,8 +281,22 @@ __global__ void __launch_bounds__(SW, strip_min_ctas(MODE, EDDY, (int)sizeof(R))
 // CTAs of a launch with sh rows per strip segment.
 int64_t fv_ctas(int nx, int ny, int sh) { return (int64_t)((nx + SO - 1) / SO) * ((ny + sh - 1) / sh); }
 
-// Rows per strip segment for a grid.  SWALS_FV_ROWS sets it.
-int fv_rows(int ctas_per_sm, int nx, int ny)
+// Rows per strip segment for a grid (SWALS_FV_ROWS sets it): the candidate
+// with the least estimate of the time a segment's CTAs take,
+//   (rows + 2) x CTA-rows that an SM works through per row of a segment.
+// The two rows stand for the lead-in, whose rows do part of a row's work.  An
+// SM runs up to five CTAs side by side; fewer than three take the time of
+// three (a row of one CTA is a serial chain: 2.6 us a row for one pass at
+// 300 x 200, against 0.76 us a CTA-row on full SMs); CTAs beyond the five
+// follow as others end, which hides most of a last, smaller round.
+// Measured on the B200, a step in us, the estimate's rows against the best
+// of 1 .. 32 and the 8 or 12 taken before: rk2 FP64 120 x 80 1 row 32.0
+// (8 rows 71.0), 300 x 200 2: 42.6 (8: 71.0), 520 x 390 5: 66.1 (4: 65.0,
+// 8: 78.0), 930^2 14: 160.3 (5: 156.4, 8: 172.0), 1275 x 879 14: 198.1
+// (7: 192.4, 12: 216.2), 2048^2 16: 556.5 (12: 557.9); midpoint 930^2 14:
+// 144.2 (8: 152.5).  Over 20 grids, methods and both precisions 1.4 % above
+// the best on average, 5.5 % at most.
+int fv_rows(int nx, int ny)
 {
     const char *e = getenv("SWALS_FV_ROWS");
     if (e && atoi(e) > 0) return atoi(e);
@@ -292,14 +306,21 @@ int fv_rows(int ctas_per_sm, int nx, int ny)
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         sms = n;
     }
-    const int slots = ctas_per_sm * sms;   // resident CTAs
-    const int cand[] = {12, 16, 8, 24};
+    const int cand[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16};
+    constexpr double resident = 5.0, chain = 3.0, exposed = 0.3;
     int best = 0;
     double best_cost = 0.0;
     for (int sh : cand) {
-        const double w = (double)fv_ctas(nx, ny, sh) / slots;
-        const double cost = (sh + 4.0) / sh * std::ceil(w) / w;
-        if (best == 0 || cost < 0.98 * best_cost) {
+        const double ctas = (double)fv_ctas(nx, ny, sh) / sms;
+        double w;
+        if (ctas <= resident) {
+            w = std::fmax(chain, std::ceil(ctas));
+        } else {
+            const double rest = std::fmod(ctas, resident);
+            w = ctas + (rest > 0.0 ? exposed * std::fmax(chain - rest, 0.0) : 0.0);
+        }
+        const double cost = (sh + 2.0) * w;
+        if (best == 0 || cost < best_cost) {
             best = sh;
             best_cost = cost;
         }
@@ -315,7 +336,7 @@ cudaError_t launch_stage_stream(const Rk2Args<R> &a, cudaStream_t s)
     // Stage 2 takes the first stage's dt and accumulates no CFL maximum: its
     // kernels leave the edges' wave-speed candidates out.
     if (MODE == MODE_STAGE2 && a.write_cfl) return cudaErrorInvalidValue;
-    const int SH = fv_rows(4, a.nx, a.ny);
+    const int SH = fv_rows(a.nx, a.ny);
     const int blocks = (int)fv_ctas(a.nx, a.ny, SH);
     if constexpr (MODE != MODE_CFL) {
         if (a.flux_variant & FLUX_EDDY) {
