@@ -234,6 +234,14 @@ swals::LaunchHook swals::hook_of(swals_domain *d)
 
 namespace {
 
+void make_aux(swals_domain *d)
+{
+    if (d->aux.stream) return;
+    cudaStreamCreateWithFlags(&d->aux.stream, cudaStreamNonBlocking);
+    cudaEventCreateWithFlags(&d->aux.fork, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&d->aux.join, cudaEventDisableTiming);
+}
+
 template <typename R>
 int evolve_t(swals_domain *d, double timestep, int has_dt)
 {
@@ -292,11 +300,7 @@ int evolve_t(swals_domain *d, double timestep, int has_dt)
         p.stg = (const R *)d->planes[in][0]; p.uh = (const R *)d->planes[in][1]; p.vh = (const R *)d->planes[in][2];
         p.stg_o = (R *)d->planes[out][0]; p.uh_o = (R *)d->planes[out][1]; p.vh_o = (R *)d->planes[out][2];
         p.elv = (R *)d->elv; p.max_stage = max_stage; p.manning_sq = (R *)d->manning_sq;
-        if (!d->aux.stream) {
-            cudaStreamCreateWithFlags(&d->aux.stream, cudaStreamNonBlocking);
-            cudaEventCreateWithFlags(&d->aux.fork, cudaEventDisableTiming);
-            cudaEventCreateWithFlags(&d->aux.join, cudaEventDisableTiming);
-        }
+        make_aux(d);
         // the step kernel records the gauges when it is the step's last one
         StepConfig cg = c;
         cg.g_sites = d->d_sites;
@@ -585,8 +589,11 @@ int swals_gpu_domain_create(const swals_domain_desc *desc, swals_domain **out)
 
 static void drop_step_graph(swals_domain *d)
 {
-    if (d->step_graph) cudaGraphExecDestroy(d->step_graph);
-    d->step_graph = nullptr;
+    for (auto &by_cur : d->step_graph)
+        for (auto &g : by_cur) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = swals_domain::StepGraph{};
+        }
 }
 
 static void free_forcing(swals_domain *d)
@@ -621,6 +628,8 @@ int swals_gpu_domain_destroy(swals_domain *d)
     if (d->aux.stream) {
         cudaStreamSynchronize(d->aux.stream);
         cudaStreamDestroy(d->aux.stream);
+        for (cudaEvent_t e : {d->pair_main, d->pair_edge[0], d->pair_edge[1]})
+            if (e) cudaEventDestroy(e);
         cudaEventDestroy(d->aux.fork);
         cudaEventDestroy(d->aux.join);
     }
@@ -716,12 +725,139 @@ int swals_gpu_evolve_one_step(swals_domain *d, double timestep, int32_t has_time
     return d->fp64 ? evolve_t<double>(d, timestep, has_timestep) : evolve_t<float>(d, timestep, has_timestep);
 }
 
-// nsteps calls of evolve_one_step.  Long runs replay a CUDA graph of
-// GRAPH_STEPS steps (a multiple of 3, so every method's state-buffer
-// rotation returns to where it started): the sequence of launches is the
-// same, without the per-launch host cost.  Timed (timers on) and first
-// steps run one by one.
-static constexpr int GRAPH_STEPS = 6;
+}  // extern "C"
+
+namespace {
+
+// Two plain linear steps of fixed dt by one pass (linear_pair.cu), `pair`-th
+// of a sequence; their bookkeeping follows on the side stream, beside the
+// next pair.  A line buffer and a state buffer are written again two and three
+// pairs on, after the bookkeeping that reads them (pair_edge).
+template <typename R>
+swals::LinearPair<R> pair_args(swals_domain *d, double timestep, int pair)
+{
+    swals::LinearPair<R> a{};
+    const int in = d->cur, out = (d->cur + 1) % 3;
+    a.p.nx = d->nx; a.p.ny = d->ny; a.p.pitch = d->pitch;
+    a.p.stg = (const R *)d->planes[in][0]; a.p.uh = (const R *)d->planes[in][1]; a.p.vh = (const R *)d->planes[in][2];
+    a.p.stg_o = (R *)d->planes[out][0]; a.p.uh_o = (R *)d->planes[out][1]; a.p.vh_o = (R *)d->planes[out][2];
+    a.p.elv = (R *)d->elv;
+    a.p.max_stage = d->desc.record_max_stage ? (R *)d->max_stage : nullptr;
+    a.m = swals::metrics_of<R>(d);
+    a.dt = R(timestep);
+    a.nbatch = 1;
+    a.fw = (const R *)d->cfg.fw;
+    a.fw_plane = d->pitch * (int64_t)d->ny;
+    a.g_sites = d->d_sites; a.g_n = d->n_gauges; a.g_vals = 3; a.g_capacity = d->gauge_capacity;
+    a.g_rec = d->d_records;
+    a.g_count = &d->sc->gauge_records;
+    a.g_done = reinterpret_cast<unsigned *>(&d->sc->blocks_done);
+    a.lines = reinterpret_cast<R *>(d->lines) + (pair & 1) * (2 * d->nx + 2 * d->ny);
+    return a;
+}
+
+// Whether evolve_steps may take two steps at a time: a plain leapfrog step
+// (no boundary routine, forcing or changing friction work), max_stage after
+// every step or not at all.  A kernel chosen by SWALS_LINEAR_KERNEL steps
+// singly.  Both sides measured, a step in us, single / pair: see linear_pair.cu.
+bool takes_pairs(const swals_domain *d, int has_dt)
+{
+    const bool lf = d->method == M_LINEAR || (d->method == M_LF_LIN_NLFRIC && d->cfg.truely_linear);
+    if (!lf || !has_dt || d->cfg.bc_kind != SWALS_BC_NONE || d->cfg.n_forcing || d->timers_on || d->static_pending)
+        return false;
+    if (d->desc.record_max_stage && (d->max_U_update_frequency > 1 || d->max_u_generic)) return false;
+    const char *e = getenv("SWALS_LINEAR_KERNEL");
+    if (e && *e && strcmp(e, "pair") != 0) return false;
+    return d->fp64 ? swals::linear_pair_fits<double>(pair_args<double>(const_cast<swals_domain *>(d), 0.0, 0).p, 0, 0)
+                   : swals::linear_pair_fits<float>(pair_args<float>(const_cast<swals_domain *>(d), 0.0, 0).p, 0, 0);
+}
+
+template <typename R>
+int evolve_pairs_t(swals_domain *d, double timestep, int npairs)
+{
+    make_aux(d);
+    for (cudaEvent_t *e : {&d->pair_main, &d->pair_edge[0], &d->pair_edge[1]})
+        if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    const swals::LaunchHook hook = swals::hook_of(d);
+    for (int k = 0; k < npairs; k++) {
+        const swals::LinearPair<R> a = pair_args<R>(d, timestep, k);
+        if (k >= 2) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[k & 1], 0));
+        hook(swals::CAT_LINEAR_MAIN, 0);
+        CK(swals::launch_linear_pair<R>(a, d->cfg, d->stream));
+        hook(swals::CAT_LINEAR_MAIN, 1);
+        CK(cudaEventRecord(d->pair_main, d->stream));
+        CK(cudaStreamWaitEvent(d->aux.stream, d->pair_main, 0));
+        hook(swals::CAT_LINEAR_EDGE, 0);
+        CK(swals::launch_linear_pair_edge<R>(a, d->cfg, d->sc, d->aux.stream));
+        hook(swals::CAT_LINEAR_EDGE, 1);
+        CK(cudaEventRecord(d->pair_edge[k & 1], d->aux.stream));
+        d->cur = (d->cur + 1) % 3;
+        d->nsteps += 2;
+    }
+    if (npairs > 0) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[(npairs - 1) & 1], 0));
+    return SWALS_OK;
+}
+
+int evolve_pairs(swals_domain *d, double timestep, int npairs)
+{
+    return d->fp64 ? evolve_pairs_t<double>(d, timestep, npairs) : evolve_pairs_t<float>(d, timestep, npairs);
+}
+
+}  // namespace
+
+extern "C" {
+
+// nsteps calls of evolve_one_step.  Long runs replay CUDA graphs of a few
+// steps: the sequence of launches is the same, without the per-launch host
+// cost.  A graph's steps are a multiple of 6, so that every method's rotation
+// of the three state buffers, by one step or by a pair of linear steps, returns
+// to where it started; a graph reads and writes the buffers it was captured
+// with, so each starting buffer has its own.  Pairs take graphs of 24 steps
+// where they fit.  Timed (timers on) and first steps run one by one.
+static constexpr int GRAPH_STEPS[2] = {6, 24};
+
+static int step_graph(swals_domain *d, int which, double timestep, int32_t has_timestep, bool pairs)
+{
+    const bool same = d->graph_dt == timestep && d->graph_has_dt == (has_timestep != 0) && d->graph_pairs == pairs &&
+                      d->graph_stream == d->stream && d->graph_gauges == d->n_gauges;
+    if (!same) {
+        drop_step_graph(d);
+        d->graph_dt = timestep;
+        d->graph_has_dt = has_timestep != 0;
+        d->graph_pairs = pairs;
+        d->graph_stream = d->stream;
+        d->graph_gauges = d->n_gauges;
+    }
+    swals_domain::StepGraph &sg = d->step_graph[d->cur][which];
+    if (sg.exec) return SWALS_OK;
+    const int cur0 = d->cur;
+    const int64_t n0 = d->nsteps, l0 = d->launches;
+    if (pairs) {   // (created outside the capture)
+        int rc = evolve_pairs(d, timestep, 0);
+        if (rc) return rc;
+    }
+    CK(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = SWALS_OK;
+    if (pairs) {
+        rc = evolve_pairs(d, timestep, GRAPH_STEPS[which] / 2);
+    } else {
+        for (int s = 0; s < GRAPH_STEPS[which] && rc == SWALS_OK; s++)
+            rc = d->fp64 ? evolve_t<double>(d, timestep, has_timestep) : evolve_t<float>(d, timestep, has_timestep);
+    }
+    cudaGraph_t g = nullptr;
+    cudaError_t ce = cudaStreamEndCapture(d->stream, &g);
+    const bool back = (d->cur == cur0);
+    sg.launches = d->launches - l0;
+    d->cur = cur0;
+    d->nsteps = n0;
+    d->launches = l0;
+    if (rc) { if (g) cudaGraphDestroy(g); return rc; }
+    if (ce != cudaSuccess) { if (g) cudaGraphDestroy(g); return cuda_fail(ce, "cudaStreamEndCapture"); }
+    if (back) ce = cudaGraphInstantiate(&sg.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ce != cudaSuccess) return cuda_fail(ce, "cudaGraphInstantiate");
+    return SWALS_OK;   // (no graph when the buffers do not come back: the steps run one by one)
+}
 
 int swals_gpu_evolve_steps(swals_domain *d, int32_t nsteps, double timestep, int32_t has_timestep)
 {
@@ -734,51 +870,30 @@ int swals_gpu_evolve_steps(swals_domain *d, int32_t nsteps, double timestep, int
         }
         return (int)SWALS_OK;
     };
-    if (d->nsteps == 0 && nsteps > 0) {
+    const bool pairs = takes_pairs(d, has_timestep);
+    if (nsteps > 0 && (d->nsteps == 0 || (pairs && d->cfg.fw && !d->cfg.fw_ready))) {
         int rc = eager(1);
         if (rc) return rc;
         done = 1;
     }
-    const bool use_graph = !d->timers_on && !d->static_pending && (nsteps - done) >= 2 * GRAPH_STEPS;
-    if (use_graph) {
-        // The graph reads and writes the state buffers it was captured
-        // with: it is valid only while the step sequence starts from the
-        // same buffer (steps taken one by one in between rotate it).
-        const bool same = d->step_graph && d->graph_dt == timestep && d->graph_has_dt == (has_timestep != 0) &&
-                          d->graph_stream == d->stream && d->graph_gauges == d->n_gauges && d->graph_cur == d->cur;
-        if (!same) {
-            drop_step_graph(d);
-            const int cur0 = d->cur;
-            const int64_t n0 = d->nsteps, l0 = d->launches;
-            CK(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal));
-            int rc = SWALS_OK;
-            for (int s = 0; s < GRAPH_STEPS && rc == SWALS_OK; s++)
-                rc = d->fp64 ? evolve_t<double>(d, timestep, has_timestep) : evolve_t<float>(d, timestep, has_timestep);
-            cudaGraph_t g = nullptr;
-            cudaError_t ce = cudaStreamEndCapture(d->stream, &g);
-            const bool back = (d->cur == cur0);
-            d->graph_launches = d->launches - l0;
-            d->cur = cur0;
-            d->nsteps = n0;
-            d->launches = l0;
-            if (rc) { if (g) cudaGraphDestroy(g); return rc; }
-            if (ce != cudaSuccess) { if (g) cudaGraphDestroy(g); return cuda_fail(ce, "cudaStreamEndCapture"); }
-            if (!back) { cudaGraphDestroy(g); return eager(nsteps - done); }
-            ce = cudaGraphInstantiate(&d->step_graph, g, 0);
-            cudaGraphDestroy(g);
-            if (ce != cudaSuccess) return cuda_fail(ce, "cudaGraphInstantiate");
-            d->graph_dt = timestep;
-            d->graph_has_dt = has_timestep != 0;
-            d->graph_stream = d->stream;
-            d->graph_gauges = d->n_gauges;
-            d->graph_cur = d->cur;
+    if (!d->timers_on && !d->static_pending && (nsteps - done) >= 2 * GRAPH_STEPS[0]) {
+        while (nsteps - done >= GRAPH_STEPS[0]) {
+            const int which = (pairs && nsteps - done >= GRAPH_STEPS[1]) ? 1 : 0;
+            int rc = step_graph(d, which, timestep, has_timestep, pairs);
+            if (rc) return rc;
+            const swals_domain::StepGraph &sg = d->step_graph[d->cur][which];
+            if (!sg.exec) break;
+            CK(cudaGraphLaunch(sg.exec, d->stream));
+            d->nsteps += GRAPH_STEPS[which];
+            d->launches += sg.launches;
+            done += GRAPH_STEPS[which];
         }
-        while (nsteps - done >= GRAPH_STEPS) {
-            CK(cudaGraphLaunch(d->step_graph, d->stream));
-            d->nsteps += GRAPH_STEPS;
-            d->launches += d->graph_launches;
-            done += GRAPH_STEPS;
-        }
+    }
+    if (pairs && nsteps - done >= 2) {
+        const int n = (nsteps - done) / 2;
+        int rc = evolve_pairs(d, timestep, n);
+        if (rc) return rc;
+        done += 2 * n;
     }
     return eager(nsteps - done);
 }

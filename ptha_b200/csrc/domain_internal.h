@@ -68,14 +68,16 @@ struct swals_domain {
     swals::MaxUConfig max_u{};     // optional max_U_variables (planes nx x ny, allocated when set)
     bool max_u_generic = false;     // max_stage and the options by max_u_kernel instead of the step kernels
     size_t stage_cap = 0;
-    // Replayed graph of a few steps for evolve_steps.
-    cudaGraphExec_t step_graph = nullptr;
+    // Replayed graphs of a few steps for evolve_steps, by the state buffer
+    // they start from (and return to) and by length.
+    struct StepGraph { cudaGraphExec_t exec = nullptr; int64_t launches = 0; };
+    StepGraph step_graph[3][2];
     double graph_dt = 0.0;
-    bool graph_has_dt = false;
+    bool graph_has_dt = false, graph_pairs = false;
     cudaStream_t graph_stream = nullptr;
     int graph_gauges = -1;
-    int graph_cur = -1;            // state buffer the graph starts from (and returns to)
-    int64_t graph_launches = 0;
+    // Pairs of linear steps: the pair kernel's end, each line buffer's reader's end.
+    cudaEvent_t pair_main = nullptr, pair_edge[2] = {};
     // misfit_gradient's replayed graphs (segments of K steps), valid for
     // (adj_K, adj_ng, adj_dt, ws).
     // [0] forward; [1 + 3 set] recompute into buffer set `set`;

@@ -160,6 +160,41 @@ template <typename R>
 cudaError_t launch_linear_map(const StepPlanes<R> &p, const Metrics<R> &m, const StepConfig &c, R dt,
                               const int *sites, int n_sites, double *rec, cudaStream_t s, const LaunchHook &hook);
 
+// Two linear leapfrog steps in one pass (linear_pair.cu): p's output planes
+// hold the state two steps on.  Plain steps only (no boundary routine, no
+// forcing), on planes that linear_pair_fits accepts.  The caller fills the
+// members up to `lines`; launch_linear_pair takes the rest from the
+// configuration.  For a plain domain the momenta of the first step on the
+// boundary-flux lines go to `lines` (N[nx], E[ny], S[nx], W[ny]) for
+// launch_linear_pair_edge, which does both steps' bookkeeping.
+template <typename R>
+struct LinearPair {
+    StepPlanes<R> p;        // planes of instance 0
+    Metrics<R> m;
+    R dt;
+    int nbatch;             // instances sharing ELV and the metrics (1 for a plain domain)
+    int64_t inst_stride, max_stride;   // elements between instances' planes, max_stage planes
+    const R *fw;            // friction work (UH points, then fw_plane elements on the VH points) or null
+    int64_t fw_plane;
+    // Gauges: sites (i, j), record (count + step) of each instance, g_vals = 3
+    // (stage, UH, VH) or 1 (stage) values; the last CTA adds two to *g_count.
+    // A null g_count stands for 0 and is not advanced.
+    const int *g_sites;
+    int g_n, g_vals, g_capacity;
+    double *g_rec;
+    int *g_count;
+    unsigned *g_done;
+    R *lines;               // null: no boundary-flux lines
+    int xl, xu, yl, yu, n_ext, lin_fric;
+    R msl, lin_fric_mult, lin_fric_dt;
+};
+template <typename R>
+bool linear_pair_fits(const StepPlanes<R> &p, int64_t inst_stride, int64_t max_stride);
+template <typename R>
+cudaError_t launch_linear_pair(LinearPair<R> a, const StepConfig &c, cudaStream_t s);
+template <typename R>
+cudaError_t launch_linear_pair_edge(const LinearPair<R> &a, const StepConfig &c, DevScalars *sc, cudaStream_t s);
+
 // Batched truly/not-truly linear leapfrog: `nbatch` instances whose planes
 // follow instance 0's at `inst_stride` elements, sharing ELV and metrics
 // (no boundary routine).  tile_cfg selects one of linear_tile_config_count()
