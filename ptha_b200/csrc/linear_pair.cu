@@ -28,7 +28,7 @@
 // 212 / 118, 8192^2 791 / 421 (a pair moves 72 B a cell: 5.1 and 5.7
 // TB/s, 0.79 and 0.89 of the copy bandwidth), 3600 x 2400 FP32 Coriolis 71.8 /
 // 43.6, 1200 x 800 Coriolis 20.5 / 12.2, 400^2 with 9 gauges 9.2 / 6.4, 200 x
-// 150 9.3 / 4.9; with Manning friction 1501 x 1001 Coriolis 58.3 / 52.3.
+// 150 9.3 / 4.9; with Manning friction 1501 x 1001 Coriolis 58.1 / 29.3.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -52,6 +52,12 @@ __device__ __forceinline__ void cp16(void *smem, const void *gmem, int src_bytes
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(src_bytes));
 }
 
+// CTAs per SM the register cap is sized for.  With the friction work the two
+// steps' square roots and quotients bind, not the memory, and spills cost more
+// than warps: 1501 x 1001 FP64 Coriolis 52.3 us a step at 4 (spilling), 29.5
+// at 3, 29.3 at 2 (188 registers); FP32 3000 x 2000 95 / 77 / 77.
+constexpr int pair_ctas(bool nlf, int real_bytes) { return !nlf ? 4 : real_bytes == 8 ? 2 : 3; }
+
 // Row constants of a segment, rows ra - 2 .. (clamped to the grid).
 template <typename R> struct RowConst {
     R cs, cu, cv, dxb, dxb1, dtc, dtj;   // dt/area, g dt/area, g dt/mean area, distance_bottom_edge(r), (r+1), dt cor/2 ...
@@ -71,7 +77,7 @@ __device__ __forceinline__ float friction_multiplier(float lf1, float dt, float 
 }
 
 template <typename R, bool COR, bool TL, bool NLF, bool GAUGES>
-__global__ void __launch_bounds__(32 * WPC, 4) linear_pair_kernel(const LinearPair<R> a, int SH, int nstrips)
+__global__ void __launch_bounds__(32 * WPC, pair_ctas(NLF, (int)sizeof(R))) linear_pair_kernel(const LinearPair<R> a, int SH, int nstrips)
 {
     constexpr int CPL = 16 / (int)sizeof(R);
     constexpr int OUTC = 30 * CPL;
@@ -463,7 +469,9 @@ __global__ void __launch_bounds__(512) linear_pair_edge_kernel(const LinearPair<
 // rows (best of 4 .. 64): 200 x 150 FP64 4: 4.9; 400^2 4: 6.4; 1200 x 800
 // Coriolis 8: 12.2 (16: 11.8); 4096^2 64: 118.1 (24: 112.7); 8192^2 48:
 // 420.7; 3600 x 2400 FP32 Coriolis 48: 43.6.
-int pair_rows(int64_t groups, int ny, int nbatch)
+// The friction form runs two (FP32 three) CTAs an SM in equal rounds: 24 rows
+// at 1501 x 1001, the best there.
+int pair_rows(int64_t groups, int ny, int nbatch, int rounds_of)
 {
     const char *e = getenv("SWALS_PAIR_ROWS");
     if (e && atoi(e) > 0) return std::min(atoi(e), 256);
@@ -479,7 +487,9 @@ int pair_rows(int64_t groups, int ny, int nbatch)
     for (int sh : {4, 6, 8, 12, 16, 24, 32, 48, 64}) {
         const double ctas = (double)groups * nbatch * ((ny + sh - 1) / sh) / sms;
         double w;
-        if (ctas <= resident) {
+        if (rounds_of) {
+            w = rounds_of * std::ceil(ctas / rounds_of);
+        } else if (ctas <= resident) {
             w = std::max(chain, std::ceil(ctas));
         } else {
             const double rest = std::fmod(ctas, resident);
@@ -500,7 +510,7 @@ cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
     constexpr int CPL = 16 / (int)sizeof(R);
     const int nstrips = (a.p.nx + 30 * CPL - 1) / (30 * CPL);
     const int64_t groups = (nstrips + WPC - 1) / WPC;
-    const int sh = pair_rows(groups, a.p.ny, a.nbatch);
+    const int sh = pair_rows(groups, a.p.ny, a.nbatch, NLF ? pair_ctas(NLF, (int)sizeof(R)) : 0);
     const int64_t ctas = groups * ((a.p.ny + sh - 1) / sh) * a.nbatch;
     const size_t smem = 16 * 32 * (NLF ? 7 : 5) * SLOTS * WPC + sizeof(RowConst<R>) * (sh + 4);
     auto go = [&](auto kernel) -> cudaError_t {
