@@ -497,6 +497,48 @@ cudaError_t map_step(swals_domain *d, R *const in[3], R *const out[3], double dt
                                        stream ? stream : d->stream, swals::hook_of(d));
 }
 
+// Two such updates in one pass (linear_pair.cu), the gauge stage of both into
+// rec[0 .. ng), rec[ng .. 2 ng).
+template <typename R>
+swals::LinearPair<R> pair_args(swals_domain *d, R *const in[3], R *const out[3], double dt, const int *sites, int ng,
+                               double *rec)
+{
+    swals::LinearPair<R> a{};
+    a.p.nx = d->nx; a.p.ny = d->ny; a.p.pitch = d->pitch;
+    a.p.stg = in[0]; a.p.uh = in[1]; a.p.vh = in[2];
+    a.p.stg_o = out[0]; a.p.uh_o = out[1]; a.p.vh_o = out[2];
+    a.p.elv = (R *)d->elv;
+    a.m = swals::metrics_of<R>(d);
+    a.dt = R(dt);
+    a.nbatch = 1;
+    if (rec) { a.g_sites = sites; a.g_n = ng; a.g_vals = 1; a.g_capacity = 2; a.g_rec = rec; }
+    return a;
+}
+
+// `count` updates of the state in x[c], by pairs where the planes allow it;
+// returns the buffer they end in.  An even count ends where it began, so that
+// a graph of it can be replayed: after an odd number of pairs the last two
+// updates are single ones.  rec: count x ng gauge stages, or null.
+template <typename R>
+int map_steps(swals_domain *d, R *const x[2][3], int c, int count, double dt, const int *sites, int ng, double *rec,
+              cudaStream_t stream, cudaError_t &err)
+{
+    const swals::LaunchHook hook = swals::hook_of(d);
+    const swals::LinearPair<R> probe = pair_args<R>(d, x[0], x[1], dt, nullptr, 0, nullptr);
+    int pairs = swals::linear_pair_fits<R>(probe.p, 0, 0) ? count / 2 : 0;
+    if (count % 2 == 0 && pairs % 2 == 1) pairs--;
+    int n = 0;
+    for (int k = 0; k < pairs && err == cudaSuccess; k++, n += 2, c = 1 - c) {
+        hook(swals::CAT_LINEAR_MAIN, 0);
+        err = swals::launch_linear_pair<R>(pair_args<R>(d, x[c], x[1 - c], dt, sites, ng, rec ? rec + (size_t)n * ng : nullptr),
+                                           d->cfg, stream);
+        hook(swals::CAT_LINEAR_MAIN, 1);
+    }
+    for (; n < count && err == cudaSuccess; n++, c = 1 - c)
+        err = map_step<R>(d, x[c], x[1 - c], dt, rec ? sites : nullptr, rec ? ng : 0, rec ? rec + (size_t)n * ng : nullptr, stream);
+    return c;
+}
+
 // Residuals of `count` recorded steps against the target, and each step's
 // half squared misfit (the loss is summed over steps in forward order at
 // the end, so it does not depend on the checkpoint spacing).
@@ -583,22 +625,16 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     // The per-segment step sequences.  For an even K a full segment leaves
     // the buffer parity unchanged, so each sequence is captured once as a
     // CUDA graph and replayed for every full segment.
-    auto fwd_seq = [&](int count) {   // xs[0][0] -> xs[0][0] after an even count
-        int c = 0;
-        for (int n = 0; n < count; n++) {
-            ck(map_step<R>(d, xs[0][c], xs[0][1 - c], dt, nullptr, 0, nullptr), "forward");
-            c = 1 - c;
-        }
+    auto fwd_seq = [&](int count, int c) {   // from xs[0][c]; back there after an even count
+        cudaError_t err = cudaSuccess;
+        c = map_steps<R>(d, xs[0], c, count, dt, nullptr, 0, nullptr, d->stream, err);
+        ck(err, "forward");
         return c;
     };
     auto rec_seq = [&](int count, int set, cudaStream_t st) {   // recompute, recording the gauge stage
-        int c = 0;
-        for (int n = 0; n < count; n++) {
-            ck(map_step<R>(d, xs[set][c], xs[set][1 - c], dt, d_sites, ng, d_rec[set] + (size_t)n * ng, st),
-               "recompute");
-            c = 1 - c;
-        }
-        return c;
+        cudaError_t err = cudaSuccess;
+        map_steps<R>(d, xs[set], 0, count, dt, d_sites, ng, d_rec[set], st, err);
+        ck(err, "recompute");
     };
     auto adj_seq = [&](int count, int lc, int set) {   // adjoint back through `count` steps
         for (int t = count; t > 0; t--) {
@@ -616,7 +652,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
         const int64_t l0 = d->launches;
         for (int q = 0; q < 7 && rc == SWALS_OK; q++) {
             ck(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal), "capture");
-            if (q == 0) fwd_seq(K);
+            if (q == 0) fwd_seq(K, 0);
             else if ((q - 1) % 3 == 0) rec_seq(K, (q - 1) / 3, d->stream);
             else adj_seq(K, (q - 2) % 3, (q - 2) / 3);
             cudaGraph_t gr = nullptr;
@@ -630,24 +666,20 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
         if (rc == SWALS_OK) { d->adj_K = K; d->adj_ng = ng; d->adj_dt = dt; d->adj_ws = d->ws; }
     }
 
-    // Forward sweep with checkpoints (every segment starts in xs[0][0]).
+    // Forward sweep with checkpoints, up to the last one: nothing reads the
+    // states after it but its own recomputation.
     int cur = 0;
     for (int sgm = 0; sgm < nseg && rc == SWALS_OK; sgm++) {
         const int n0 = sgm * K, cnt = (n0 + K < nsteps) ? K : nsteps - n0;
         for (int v = 0; v < 3; v++)
             ck(cudaMemcpyAsync(ckpt + ((size_t)sgm * 3 + v) * plane, xs[0][cur][v], plane * es,
                                cudaMemcpyDeviceToDevice, d->stream), "checkpoint");
+        if (sgm == nseg - 1) break;
         if (graphs && cnt == K && cur == 0) {
             ck(cudaGraphLaunch(d->adj_graph[0], d->stream), "forward graph");
             d->launches += K;
         } else {
-            // A last, shorter segment (no state is needed after it).
-            int c = cur;
-            for (int n = 0; n < cnt; n++) {
-                ck(map_step<R>(d, xs[0][c], xs[0][1 - c], dt, nullptr, 0, nullptr), "forward");
-                c = 1 - c;
-            }
-            cur = c;
+            cur = fwd_seq(cnt, cur);
         }
     }
     // Recompute segment sgm into buffer set `set` on stream st, then its residuals.
