@@ -322,7 +322,9 @@ int evolve_t(swals_domain *d, double timestep, int has_dt)
         p.stg = (const R *)d->planes[in][0]; p.uh = (const R *)d->planes[in][1]; p.vh = (const R *)d->planes[in][2];
         p.stg_o = (R *)d->planes[out][0]; p.uh_o = (R *)d->planes[out][1]; p.vh_o = (R *)d->planes[out][2];
         p.elv = (R *)d->elv; p.max_stage = max_stage; p.manning_sq = (R *)d->manning_sq;
-        e = launch_leapfrog_nonlinear_step<R>(p, m, c, R(timestep), d->sc, d->stream, hook);
+        make_aux(d);
+        e = launch_leapfrog_nonlinear_step<R>(p, m, c, R(timestep), d->sc, d->stream, hook,
+                                              d->timers_on ? nullptr : &d->aux);
         if (e != cudaSuccess) return cuda_fail(e, "nonlinear leapfrog step");
         d->cur = out;
     } else if (d->method == M_RK2 || d->method == M_EULER || d->method == M_MIDPOINT || d->method == M_RK2N) {
@@ -532,10 +534,10 @@ int swals_gpu_domain_create(const swals_domain_desc *desc, swals_domain **out)
                                d->method == M_RK2N)
                                   ? al((size_t)swals::rk2_edge_bytes(d->pitch, ny, (int)es)) : 0;
     total += edge_bytes;
-    const size_t fw_bytes = (d->method == M_LF_LIN_NLFRIC || d->method == M_LF_NONLINEAR) ? 2 * al(plane) : 0;
+    const size_t fw_bytes = (d->method == M_LF_LIN_NLFRIC) ? 2 * al(plane) : 0;
     total += fw_bytes;   // friction_work
-    const size_t nl_bytes = (d->method == M_LF_NONLINEAR) ? 9 * al((size_t)d->pitch * (ny + 1) * es) : 0;
-    total += nl_bytes;   // leapfrog_nonlinear work planes
+    const size_t nl_bytes = (d->method == M_LF_NONLINEAR) ? al((size_t)d->pitch * (ny + 1) * es) : 0;
+    total += nl_bytes;   // leapfrog_nonlinear: the depth before the step
     e = cudaMalloc(&d->pool, total);
     if (e != cudaSuccess) {
         cudaStreamDestroy(d->stream);

@@ -2019,22 +2019,31 @@ cudaError_t launch_linear_step(const StepPlanes<R> &p, const Metrics<R> &m, cons
 // leapfrog's stage sweep, boundary and forcing, then upwind advection of the
 // momenta from a lagged depth, the momentum update with nonlinear pressure
 // gradient, Coriolis, spherical metric terms and semi-implicit friction, and
-// the dry-cell outflow limiter.  A secondary solver: one kernel per stage of
-// the reference's algorithm, reading the old momenta throughout (the
-// reference's row carries and thread-boundary copies only serve that).
-// Work planes (pitch P): lag0, advection UUH, UVH, VUH, VVH, fluxes
-// EW-UH, NS-UH, NS-VH, EW-VH (ny + 1 rows each).
+// the dry-cell outflow limiter.
+//
+// Two passes over the grid: the stage sweep (with max_stage when nothing
+// changes the stage after it), then, per tile in shared memory, the lagged
+// depths, the advection terms, the upwind fluxes and the momenta with the
+// friction work and the outflow limiter.  One kernel per stage of the
+// reference's algorithm wrote and read back nine work planes and took 86 us a
+// step at 1024 x 768 FP64; the two take 50, bound by the latency of the second
+// one's loads and divisions (40 % of the issue slots).
 namespace nl {
+
+// Tile and CTAs per SM, 1024 x 768 / 2000 x 1800 FP64, us a step: 32 x 16 and
+// 3 CTAs 54.2 / 267, 4 52.5 / 243; 32 x 8 and 3 56.8 / 301, 4 50.9 / 253, 5
+// 50.2 / 240 (200 x 150 10.7, 32 x 16 14.3).
+constexpr int TX = 32, TY = 8, NT = 256;
 
 template <typename R> struct NLArgs {
     LinArgs<R> a;
     const R *nsq;
-    R *lag0;
-    R *adv[4];      // UUH, UVH, VUH, VVH
-    R *flx[4];      // EW-UH, NS-UH, NS-VH, EW-VH
-    const R *fw;    // friction_work, UH then VH plane
-    int64_t plane;  // elements per work plane
+    R *lag0;        // depth before the step, or null: taken from the old stage
+    int chezy;
 };
+
+template <typename R>
+__device__ __forceinline__ R positive(R d) { return (R(0) > d) ? R(0) : d; }
 
 template <typename R>
 __device__ __forceinline__ bool wet(const NLArgs<R> &n, int i, int r)
@@ -2049,10 +2058,10 @@ template <typename R>
 __device__ __forceinline__ R lag(const NLArgs<R> &n, int i, int r)
 {
     const int64_t o = (int64_t)r * n.a.p.pitch + i;
-    const R d0 = n.lag0[o];
+    const R e = n.a.p.elv[o];
+    const R d0 = n.lag0 ? n.lag0[o] : positive(n.a.p.stg[o] - e);
     if (r > n.a.p.ny - 2) return d0;
-    const R dn = n.a.p.stg_o[o] - n.a.p.elv[o];
-    return K<R>::half() * (d0 + ((R(0) > dn) ? R(0) : dn));
+    return K<R>::half() * (d0 + positive(n.a.p.stg_o[o] - e));
 }
 
 template <typename R>
@@ -2061,250 +2070,289 @@ __global__ void lag0_kernel(NLArgs<R> n)
     const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
     if (i >= n.a.p.nx || r >= n.a.p.ny) return;
     const int64_t o = (int64_t)r * n.a.p.pitch + i;
-    const R dp = n.a.p.stg[o] - n.a.p.elv[o];
-    n.lag0[o] = (R(0) > dp) ? R(0) : dp;   // max(depth, 0)
+    n.lag0[o] = positive(n.a.p.stg[o] - n.a.p.elv[o]);   // max(depth, 0)
 }
 
+// max_stage: the plane to update with the new stage over xl..xu, yl..yu, or null.
 template <typename R>
-__global__ void stage_kernel(NLArgs<R> n)
+__global__ void stage_kernel(NLArgs<R> n, R *max_stage, int xl, int xu, int yl, int yu)
 {
     const LinArgs<R> &a = n.a;
     const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
     if (i >= a.p.nx || r >= a.p.ny) return;
     const int64_t o = (int64_t)r * a.p.pitch + i;
     const bool interior = (i >= 1) && (i <= a.p.nx - 2) && (r >= 1) && (r <= a.p.ny - 2);
-    if (interior) a.p.stg_o[o] = swept_stage(a, i, r);
-    else if (!(a.bc_stage && on_bc_ring(i, r, a.p.nx, a.p.ny, a.bext))) a.p.stg_o[o] = a.p.stg[o];
+    R s;
+    if (interior) s = swept_stage(a, i, r);
+    else if (a.bc_stage && on_bc_ring(i, r, a.p.nx, a.p.ny, a.bext)) s = a.p.stg_o[o];
+    else s = a.p.stg[o];
+    a.p.stg_o[o] = s;
+    if (max_stage && i >= xl && i <= xu && r >= yl && r <= yu) {
+        const R m = max_stage[o];
+        max_stage[o] = (s > m) ? s : m;
+    }
 }
 
-// The advection terms with the reference's edge extrapolations folded in
-// as index remaps (:236-333).
-template <typename R>
-__global__ void advection_kernel(NLArgs<R> n)
+// The advection terms at (i, r) with the reference's edge extrapolations
+// folded in as index remaps (:236-333): UUH, UVH at (i+1/2, j), rows
+// 0..ny-2, the last row copying row ny-2; VVH at (i, j+1/2), rows 0..ny-2;
+// VUH rows 0..ny-3 and columns 1.., the rest copied from column 1 and row
+// ny-3.
+// lag(i, r): the lagged depth.
+template <typename R> struct Adv { R uuh, uvh, vuh, vvh; };
+template <typename R, typename Lag>
+__device__ __forceinline__ Adv<R> advection(const NLArgs<R> &n, int i, int r, Lag lag)
 {
     const int nx = n.a.p.nx, ny = n.a.p.ny;
-    const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
-    if (i >= nx || r >= ny) return;
-    const int64_t P = n.a.p.pitch, o = (int64_t)r * P + i;
+    const int64_t P = n.a.p.pitch;
     const R half = K<R>::half(), mad = K<R>::min_depth(), quarter = R(0.25);
     const R *uh = n.a.p.uh, *vh = n.a.p.vh;
-    auto inv_d = [&](R dl) -> R { return (dl > mad) ? R(1) / dl : R(0); };
-    // UUH, UVH at (i+1/2, j), rows 0..ny-2; the last row copies row ny-2
+    auto inv_d = [&](R dl) -> R { return (dl > mad) ? depth_inverse(dl) : R(0); };
+    Adv<R> w;
+    const int rr = (r <= ny - 2) ? r : ny - 2;
     {
-        const int rr = (r <= ny - 2) ? r : ny - 2;
         const int jm1 = (rr - 1 > 0) ? rr - 1 : 0;
         const int iu = (i <= nx - 2) ? i : nx - 2;
         const int64_t ou = (int64_t)rr * P + iu;
-        const R dl = half * (lag(n, iu, rr) + lag(n, iu + 1, rr));
-        n.adv[0][o] = (uh[ou] * uh[ou]) * inv_d(dl);
+        const R du = inv_d(half * (lag(iu, rr) + lag(iu + 1, rr)));
+        w.uuh = (uh[ou] * uh[ou]) * du;
         const int iv = (i <= nx - 3) ? i : nx - 3;
         const int64_t ov = (int64_t)rr * P + iv;
-        const R dv = half * (lag(n, iv, rr) + lag(n, iv + 1, rr));
-        n.adv[1][o] = uh[ov] * inv_d(dv) * quarter *
-                      (vh[(int64_t)jm1 * P + iv] + vh[(int64_t)jm1 * P + iv + 1] + vh[ov] + vh[ov + 1]);
+        const R dv = (iv == iu) ? du : inv_d(half * (lag(iv, rr) + lag(iv + 1, rr)));
+        w.uvh = uh[ov] * dv * quarter *
+                (vh[(int64_t)jm1 * P + iv] + vh[(int64_t)jm1 * P + iv + 1] + vh[ov] + vh[ov + 1]);
     }
-    // VVH at (i, j+1/2), rows 0..ny-2; VUH rows 0..ny-3 and columns 1..,
-    // the rest copied from column 1 and row ny-3
     {
-        const int rr = (r <= ny - 2) ? r : ny - 2;
         const int64_t ov = (int64_t)rr * P + i;
-        const R dl = half * (lag(n, i, rr) + lag(n, i, rr + 1));
-        n.adv[3][o] = vh[ov] * vh[ov] * inv_d(dl);
+        const R dl = inv_d(half * (lag(i, rr) + lag(i, rr + 1)));
+        w.vvh = vh[ov] * vh[ov] * dl;
         const int ru = (r <= ny - 3) ? r : ny - 3;
         const int iu = (i >= 1) ? i : 1;
         const int64_t ou = (int64_t)ru * P + iu;
-        const R du = half * (lag(n, iu, ru) + lag(n, iu, ru + 1));
-        n.adv[2][o] = vh[ou] * inv_d(du) * quarter * (uh[ou - 1] + uh[ou] + uh[ou - 1 + P] + uh[ou + P]);
+        const R du = (ru == rr && iu == i) ? dl : inv_d(half * (lag(iu, ru) + lag(iu, ru + 1)));
+        w.vuh = vh[ou] * du * quarter * (uh[ou - 1] + uh[ou] + uh[ou - 1 + P] + uh[ou + P]);
     }
+    return w;
 }
 
-// Upwind fluxes of UH and VH (:340-498).  Flux planes have ny + 1 rows.
-template <typename R>
-__global__ void flux_kernel(NLArgs<R> n)
-{
-    const int nx = n.a.p.nx, ny = n.a.p.ny;
-    const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
-    if (i > nx || r > ny) return;
-    const int64_t P = n.a.p.pitch, o = (int64_t)r * P + i;
-    const R half = K<R>::half(), zero = R(0);
-    const R *uh = n.a.p.uh, *vh = n.a.p.vh;
-    const Metrics<R> &m = n.a.m;
-    const R *UUH = n.adv[0], *UVH = n.adv[1], *VUH = n.adv[2], *VVH = n.adv[3];
-    // EW flux of UH at cell centres, rows 0..ny-2
-    if (i < nx) {
-        R f = zero;
-        if (r <= ny - 2) {
-            if (i == 0) f = UUH[o] * m.dyl[0];
-            else if (i == nx - 1) f = UUH[o] * m.dyl[nx - 1];
-            else {
-                const R sm = uh[o] + uh[o - 1];
-                f = m.dyl[i] * ((sm > zero) ? UUH[o - 1] : UUH[o]);
-                if (sm == zero) f = m.dyl[i] * half * (UUH[o - 1] + UUH[o]);
-            }
-            if (!wet(n, i, r)) f = zero;
-        }
-        n.flx[0][o] = f;
-    }
-    // NS flux of UH on the bottom edge of row r (rows jl = max(r-1,0), ju = r)
-    if (i < nx) {
-        R f = zero;
-        if (i <= nx - 2 && r <= ny - 1) {
-            const int jl = (r - 1 > 0) ? r - 1 : 0, ju = r;
-            const int64_t ol = (int64_t)jl * P + i, ou = (int64_t)ju * P + i;
-            const R sm = vh[ol] + vh[ol + 1];
-            f = m.dxb[r] * ((sm > zero) ? UVH[ol] : UVH[ou]);
-            if (sm == zero) f = m.dxb[r] * half * (UVH[ol] + UVH[ou]);
-            if (!(wet(n, i, ju) && wet(n, i + 1, ju) && wet(n, i, jl) && wet(n, i + 1, jl))) f = zero;
-        }
-        n.flx[1][o] = f;
-    }
-    // NS flux of VH on the bottom edge of row r
-    if (i < nx) {
-        R f = zero;
-        if (i <= nx - 2 && r <= ny - 1) {
-            const int jm1 = (r - 1 > 0) ? r - 1 : 0;
-            const int64_t om = (int64_t)jm1 * P + i;
-            const R w = half * (m.dxb[r] + m.dxb[r + 1]);
-            const R sm = vh[o] + vh[om];
-            f = w * ((sm > zero) ? VVH[om] : VVH[o]);
-            if (sm == zero) f = w * half * (VVH[om] + VVH[o]);
-            if (!wet(n, i, r)) f = zero;
-        }
-        n.flx[2][o] = f;
-    }
-    // EW flux of VH at the west face of column i, rows 0..ny-2; column 0
-    // takes column 1's upwind value before its tie and wet/dry treatment
-    if (i < nx) {
-        R f = zero;
-        if (r <= ny - 2) {
-            const int ic = (i >= 1) ? i : 1;
-            const int64_t oc = (int64_t)r * P + ic;
-            const R sm = uh[oc - 1] + uh[oc - 1 + P];
-            f = m.dyl[ic - 1] * ((sm > zero) ? VUH[oc - 1] : VUH[oc]);
-            if (i >= 1) {
-                if (sm == zero) f = m.dyl[i - 1] * half * (VUH[oc - 1] + VUH[oc]);
-                if (!(wet(n, i - 1, r) && wet(n, i, r) && wet(n, i - 1, r + 1) && wet(n, i, r + 1))) f = zero;
-            }
-        }
-        n.flx[3][o] = f;
-    }
-}
-
+// One CTA: a TX x TY tile.
 template <typename R, bool SPH, bool COR>
-__global__ void momentum_kernel(NLArgs<R> n)
+__global__ void __launch_bounds__(NT, 5) momentum_kernel(NLArgs<R> n)
 {
     const LinArgs<R> &a = n.a;
     const int nx = a.p.nx, ny = a.p.ny;
-    const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
-    if (i >= nx || r >= ny) return;
-    const int64_t P = a.p.pitch, o = (int64_t)r * P + i;
+    const int64_t P = a.p.pitch;
+    const int i0 = blockIdx.x * TX, r0 = blockIdx.y * TY;
     const R *uh = a.p.uh, *vh = a.p.vh, *st = a.p.stg_o, *el = a.p.elv;
-    if (i > nx - 2 || r > ny - 2) {
-        a.p.uh_o[o] = uh[o];
-        a.p.vh_o[o] = vh[o];
-        return;
-    }
+    const Metrics<R> &m = a.m;
     const R g = K<R>::gravity(), half = K<R>::half(), one = K<R>::one(), zero = K<R>::zero();
     const R mad = K<R>::min_depth();
     const R dt = a.dt;
-    const R inv_cell_area_dt = dt / a.m.area[r];
-    const R inv_cell_area_dt_g = g * inv_cell_area_dt;
-    const R inv_cell_area_dt_vh = dt / (half * (a.m.area[r] + a.m.area[r + 1]));
-    const R inv_cell_area_dt_vh_g = g * inv_cell_area_dt_vh;
-    const int64_t oe = o + 1, on = o + P;
-    R h_jph = half * ((st[on] + st[o]) - (el[on] + el[o]));
-    if (h_jph < mad) h_jph = zero;
-    R h_iph = half * ((st[oe] + st[o]) - (el[oe] + el[o]));
-    if (h_iph < mad) h_iph = zero;
-    const bool jw1 = st[on] > el[on] + mad, jw0 = st[o] > el[o] + mad;
-    const R h_jph_wet_strict = (jw1 && jw0) ? one : zero;
-    const R h_jph_wet = ((h_jph_wet_strict > zero) || (jw1 && st[on] > el[o] + mad) || (jw0 && st[o] > el[on] + mad))
-                            ? one : zero;
-    const bool iw1 = st[oe] > el[oe] + mad, iw0 = jw0;
-    const R h_iph_wet_strict = (iw1 && iw0) ? one : zero;
-    const R h_iph_wet = ((h_iph_wet_strict > zero) || (iw1 && st[oe] > el[o] + mad) || (iw0 && st[o] > el[oe] + mad))
-                            ? one : zero;
-    const int rm = (r > 0) ? r - 1 : 0, im = (i > 0) ? i - 1 : 0;
-    const R vh_iph_jmh = half * (vh[(int64_t)rm * P + i] + vh[(int64_t)rm * P + i + 1]);
-    const R vh_iph_jph = half * (vh[o] + vh[oe]);
-    const R uh_i_j = half * (uh[o] + uh[(int64_t)r * P + im]);
-    const R uh_i_jp1 = half * (uh[on] + uh[(int64_t)(r + 1) * P + im]);
-    const R u0 = uh[o], v0 = vh[o];
-    const R tv = half * (vh_iph_jmh + vh_iph_jph);
-    const R tu = half * (uh_i_j + uh_i_jp1);
-    const R fm_uh = one / ((one + a.lin_fric_dt) + dt * n.fw[o] * R(sqrt(u0 * u0 + tv * tv)));
-    const R fm_vh = one / ((one + a.lin_fric_dt) + dt * n.fw[n.plane + o] * R(sqrt(v0 * v0 + tu * tu)));
-    R u = u0 * h_iph_wet - inv_cell_area_dt_g * h_iph * h_iph_wet * (st[oe] - st[o]) * a.m.dyl[i + 1];
-    R v = v0 * h_jph_wet - inv_cell_area_dt_vh_g * h_jph * h_jph_wet * (st[on] - st[o]) * a.m.dxb[r + 1];
-    const R *F0 = n.flx[0], *F1 = n.flx[1], *F2 = n.flx[2], *F3 = n.flx[3];
-    u = u - inv_cell_area_dt * R(1) * h_iph_wet * ((F0[oe] - F0[o]) + (F1[on] - F1[o]));
-    v = v - inv_cell_area_dt_vh * R(1) * h_jph_wet * ((F3[oe] - F3[o]) + (F2[on] - F2[o]));
-    if (COR) {
-        const R dthc = dt * a.m.cor[r] * half * ((h_iph_wet_strict > zero) ? one : zero);
-        const R dthc_jph = dt * a.m.cor_be[r + 1] * half * ((h_jph_wet_strict > zero) ? one : zero);
-        u = u + dthc * (vh_iph_jmh + vh_iph_jph);
-        v = v - dthc_jph * (uh_i_j + uh_i_jp1);
-    }
-    if (SPH) {
-        R inv_depth_local = zero;
-        if (h_iph_wet_strict > zero) inv_depth_local = one / h_iph;
-        const R tan_uvh = dt * a.m.tanlat[r] * u0 * half * (vh_iph_jmh + vh_iph_jph) * inv_depth_local;
-        inv_depth_local = zero;
-        if (h_jph_wet_strict > zero) inv_depth_local = one / h_jph;
-        const R tan_uuh = dt * half * (a.m.tanlat[r] + a.m.tanlat[r + 1]) * half * (uh_i_jp1 + uh_i_j) * half *
-                          (uh_i_jp1 + uh_i_j) * inv_depth_local;
-        u = u + tan_uvh;
-        v = v - tan_uuh;
-    }
-    a.p.uh_o[o] = fm_uh * u;
-    a.p.vh_o[o] = fm_vh * v;
-}
+    // lagged depths and wet cells of rows r0-2 .. r0+TY+1, columns i0-2 .. i0+TX+1
+    // (two back for the edge extrapolations of a last, narrow tile)
+    __shared__ R LAG[TY + 4][TX + 4];
+    __shared__ unsigned char W[TY + 4][TX + 4];
+    // advection terms of rows r0-1 .. r0+TY, columns i0-1 .. i0+TX
+    __shared__ R UUH[TY + 2][TX + 2], UVH[TY + 2][TX + 2], VUH[TY + 2][TX + 2], VVH[TY + 2][TX + 2];
+    // fluxes: EW of UH and VH at the west faces of columns i0 .. i0+TX, NS of
+    // UH and VH on the bottom edges of rows r0 .. r0+TY
+    __shared__ R F0[TY][TX + 1], F3[TY][TX + 1], F1[TY + 1][TX], F2[TY + 1][TX];
 
-// No outflow from dry cells (:855-880), per face.
-template <typename R>
-__global__ void dry_outflow_kernel(NLArgs<R> n)
-{
-    const int nx = n.a.p.nx, ny = n.a.p.ny;
-    const int i = blockIdx.x * 32 + threadIdx.x, r = blockIdx.y * 8 + threadIdx.y;
-    if (i >= nx || r > ny - 2) return;
-    const int64_t P = n.a.p.pitch, o = (int64_t)r * P + i;
-    const R mad = K<R>::min_depth();
-    auto dry = [&](int64_t q) { return n.a.p.stg_o[q] < n.a.p.elv[q] + mad; };
-    R u = n.a.p.uh_o[o], v = n.a.p.vh_o[o];
-    if ((dry(o) && u > R(0)) || (i + 1 <= nx - 1 && dry(o + 1) && u < R(0))) n.a.p.uh_o[o] = R(0);
-    if ((dry(o) && v > R(0)) || (dry(o + P) && v < R(0))) n.a.p.vh_o[o] = R(0);
+    for (int q = threadIdx.x; q < (TY + 4) * (TX + 4); q += NT) {
+        const int rr = q / (TX + 4), cc = q - rr * (TX + 4);
+        const int r = r0 - 2 + rr, i = i0 - 2 + cc;
+        if (r < 0 || r >= ny || i < 0 || i >= nx) continue;
+        LAG[rr][cc] = lag(n, i, r);
+        W[rr][cc] = wet(n, i, r) ? 1 : 0;
+    }
+    __syncthreads();
+    auto is_wet = [&](int i, int r) -> bool { return W[r - r0 + 2][i - i0 + 2] != 0; };
+    for (int q = threadIdx.x; q < (TY + 2) * (TX + 2); q += NT) {
+        const int rr = q / (TX + 2), cc = q - rr * (TX + 2);
+        const int r = r0 - 1 + rr, i = i0 - 1 + cc;
+        if (r < 0 || r >= ny || i < 0 || i >= nx) continue;
+        const Adv<R> w = advection(n, i, r, [&](int li, int lr) -> R { return LAG[lr - r0 + 2][li - i0 + 2]; });
+        UUH[rr][cc] = w.uuh; UVH[rr][cc] = w.uvh; VUH[rr][cc] = w.vuh; VVH[rr][cc] = w.vvh;
+    }
+    __syncthreads();
+    auto at = [&](const R(&A)[TY + 2][TX + 2], int i, int r) -> R { return A[r - r0 + 1][i - i0 + 1]; };
+
+    // Upwind fluxes (:340-498).
+    for (int q = threadIdx.x; q < TY * (TX + 1); q += NT) {
+        const int rr = q / (TX + 1), cc = q - rr * (TX + 1);
+        const int r = r0 + rr, i = i0 + cc;
+        R f0 = zero, f3 = zero;
+        if (i < nx && r <= ny - 2) {
+            const int64_t o = (int64_t)r * P + i;
+            // EW flux of UH at cell centres
+            if (i == 0) f0 = at(UUH, 0, r) * m.dyl[0];
+            else if (i == nx - 1) f0 = at(UUH, i, r) * m.dyl[nx - 1];
+            else {
+                const R sm = uh[o] + uh[o - 1];
+                f0 = m.dyl[i] * ((sm > zero) ? at(UUH, i - 1, r) : at(UUH, i, r));
+                if (sm == zero) f0 = m.dyl[i] * half * (at(UUH, i - 1, r) + at(UUH, i, r));
+            }
+            if (!is_wet(i, r)) f0 = zero;
+            // EW flux of VH at the west face of column i; column 0 takes
+            // column 1's upwind value before its tie and wet/dry treatment
+            const int ic = (i >= 1) ? i : 1;
+            const int64_t oc = (int64_t)r * P + ic;
+            const R sm = uh[oc - 1] + uh[oc - 1 + P];
+            f3 = m.dyl[ic - 1] * ((sm > zero) ? at(VUH, ic - 1, r) : at(VUH, ic, r));
+            if (i >= 1) {
+                if (sm == zero) f3 = m.dyl[i - 1] * half * (at(VUH, i - 1, r) + at(VUH, i, r));
+                if (!(is_wet(i - 1, r) && is_wet(i, r) && is_wet(i - 1, r + 1) && is_wet(i, r + 1))) f3 = zero;
+            }
+        }
+        F0[rr][cc] = f0;
+        F3[rr][cc] = f3;
+    }
+    for (int q = threadIdx.x; q < (TY + 1) * TX; q += NT) {
+        const int rr = q / TX, cc = q - rr * TX;
+        const int r = r0 + rr, i = i0 + cc;
+        R f1 = zero, f2 = zero;
+        if (i <= nx - 2 && r <= ny - 1) {
+            const int64_t o = (int64_t)r * P + i;
+            const int jl = (r - 1 > 0) ? r - 1 : 0;
+            const int64_t ol = (int64_t)jl * P + i;
+            // NS flux of UH on the bottom edge of row r
+            R sm = vh[ol] + vh[ol + 1];
+            f1 = m.dxb[r] * ((sm > zero) ? at(UVH, i, jl) : at(UVH, i, r));
+            if (sm == zero) f1 = m.dxb[r] * half * (at(UVH, i, jl) + at(UVH, i, r));
+            if (!(is_wet(i, r) && is_wet(i + 1, r) && is_wet(i, jl) && is_wet(i + 1, jl))) f1 = zero;
+            // NS flux of VH
+            const R w = half * (m.dxb[r] + m.dxb[r + 1]);
+            sm = vh[o] + vh[ol];
+            f2 = w * ((sm > zero) ? at(VVH, i, jl) : at(VVH, i, r));
+            if (sm == zero) f2 = w * half * (at(VVH, i, jl) + at(VVH, i, r));
+            if (!is_wet(i, r)) f2 = zero;
+        }
+        F1[rr][cc] = f1;
+        F2[rr][cc] = f2;
+    }
+    __syncthreads();
+
+    for (int rr = threadIdx.x / TX; rr < TY; rr += NT / TX) {
+        const int cc = threadIdx.x % TX, r = r0 + rr, i = i0 + cc;
+        if (i >= nx || r >= ny) continue;
+        const int64_t o = (int64_t)r * P + i;
+        // No outflow from dry cells (:855-880), per face, rows 0..ny-2.
+        auto dry = [&](int64_t q) { return st[q] < el[q] + mad; };
+        auto keep = [&](R u, R v) {
+            if (r <= ny - 2) {
+                const bool d = dry(o);
+                if ((d && u > zero) || (i + 1 <= nx - 1 && dry(o + 1) && u < zero)) u = zero;
+                if ((d && v > zero) || (dry(o + P) && v < zero)) v = zero;
+            }
+            a.p.uh_o[o] = u;
+            a.p.vh_o[o] = v;
+        };
+        if (i > nx - 2 || r > ny - 2) {
+            keep(uh[o], vh[o]);
+            continue;
+        }
+        const R inv_cell_area_dt = dt / m.area[r];
+        const R inv_cell_area_dt_g = g * inv_cell_area_dt;
+        const R inv_cell_area_dt_vh = dt / (half * (m.area[r] + m.area[r + 1]));
+        const R inv_cell_area_dt_vh_g = g * inv_cell_area_dt_vh;
+        const int64_t oe = o + 1, on = o + P;
+        const R s0 = st[o], s_e = st[oe], s_n = st[on], e0 = el[o], e_e = el[oe], e_n = el[on];
+        R h_jph = half * ((s_n + s0) - (e_n + e0));
+        if (h_jph < mad) h_jph = zero;
+        R h_iph = half * ((s_e + s0) - (e_e + e0));
+        if (h_iph < mad) h_iph = zero;
+        const bool jw1 = s_n > e_n + mad, jw0 = s0 > e0 + mad;
+        const bool h_jph_wet_strict = jw1 && jw0;
+        const R h_jph_wet = (h_jph_wet_strict || (jw1 && s_n > e0 + mad) || (jw0 && s0 > e_n + mad)) ? one : zero;
+        const bool iw1 = s_e > e_e + mad, iw0 = jw0;
+        const bool h_iph_wet_strict = iw1 && iw0;
+        const R h_iph_wet = (h_iph_wet_strict || (iw1 && s_e > e0 + mad) || (iw0 && s0 > e_e + mad)) ? one : zero;
+        const int rm = (r > 0) ? r - 1 : 0, im = (i > 0) ? i - 1 : 0;
+        const R u0 = uh[o], v0 = vh[o];
+        const R vh_iph_jmh = half * (vh[(int64_t)rm * P + i] + vh[(int64_t)rm * P + i + 1]);
+        const R vh_iph_jph = half * (v0 + vh[oe]);
+        const R uh_i_j = half * (u0 + uh[(int64_t)r * P + im]);
+        const R uh_i_jp1 = half * (uh[on] + uh[(int64_t)(r + 1) * P + im]);
+        const R tv = half * (vh_iph_jmh + vh_iph_jph);
+        const R tu = half * (uh_i_j + uh_i_jp1);
+        // the friction work at the two faces (precompute_friction_work, from the new stage)
+        const R n0 = n.nsq[o];
+        auto work = [&](R s1, R e1, R n1) -> R {
+            const R d = half * (((s0 - e0) + s1) - e1);
+            const R dm = (d > mad) ? d : mad;
+            const R pw = R(n.chezy ? pow_friction<true>((double)dm)
+                                   : (double)dm < 1.0e30 ? pow_friction<false, true>((double)dm) : pow_friction<false>((double)dm));
+            return g * (half * (n0 + n1)) * pw;
+        };
+        const R fm_uh = friction_multiplier(one + a.lin_fric_dt, dt, work(s_e, e_e, n.nsq[oe]), u0, tv);
+        const R fm_vh = friction_multiplier(one + a.lin_fric_dt, dt, work(s_n, e_n, n.nsq[on]), v0, tu);
+        R u = u0 * h_iph_wet - inv_cell_area_dt_g * h_iph * h_iph_wet * (s_e - s0) * m.dyl[i + 1];
+        R v = v0 * h_jph_wet - inv_cell_area_dt_vh_g * h_jph * h_jph_wet * (s_n - s0) * m.dxb[r + 1];
+        u = u - inv_cell_area_dt * R(1) * h_iph_wet * ((F0[rr][cc + 1] - F0[rr][cc]) + (F1[rr + 1][cc] - F1[rr][cc]));
+        v = v - inv_cell_area_dt_vh * R(1) * h_jph_wet * ((F3[rr][cc + 1] - F3[rr][cc]) + (F2[rr + 1][cc] - F2[rr][cc]));
+        if (COR) {
+            const R dthc = dt * m.cor[r] * half * (h_iph_wet_strict ? one : zero);
+            const R dthc_jph = dt * m.cor_be[r + 1] * half * (h_jph_wet_strict ? one : zero);
+            u = u + dthc * (vh_iph_jmh + vh_iph_jph);
+            v = v - dthc_jph * (uh_i_j + uh_i_jp1);
+        }
+        if (SPH) {
+            R inv_depth_local = zero;
+            if (h_iph_wet_strict) inv_depth_local = one / h_iph;
+            const R tan_uvh = dt * m.tanlat[r] * u0 * half * (vh_iph_jmh + vh_iph_jph) * inv_depth_local;
+            inv_depth_local = zero;
+            if (h_jph_wet_strict) inv_depth_local = one / h_jph;
+            const R tan_uuh = dt * half * (m.tanlat[r] + m.tanlat[r + 1]) * half * (uh_i_jp1 + uh_i_j) * half *
+                              (uh_i_jp1 + uh_i_j) * inv_depth_local;
+            u = u + tan_uvh;
+            v = v - tan_uuh;
+        }
+        keep(fm_uh * u, fm_vh * v);
+    }
 }
 
 }  // namespace nl
 
 // one_leapfrog_nonlinear_step (timestepping_alternatives_include.f90:
-// 439-447) on the whole domain.  c.nl_work holds the 9 work planes of
-// pitch x (ny + 1) elements; c.fw the friction work.
+// 439-447) on the whole domain.  c.nl_work (pitch x (ny + 1) elements) takes
+// the depth before the step where a boundary routine or forcing may change
+// what it is formed from.
 template <typename R>
 cudaError_t launch_leapfrog_nonlinear_step(const StepPlanes<R> &p, const Metrics<R> &m, const StepConfig &c, R dt,
-                                           DevScalars *sc, cudaStream_t s, const LaunchHook &hook)
+                                           DevScalars *sc, cudaStream_t s, const LaunchHook &hook, const AuxStream *aux)
 {
     LinArgs<R> a = make_args<R>(p, m, c, dt);
     a.xl = 0; a.xu = p.nx - 1; a.yl = 0; a.yu = p.ny - 1;   // the reference fixes the whole domain
+    // Without a boundary routine or forcing nothing changes the stage after
+    // its sweep, nor the old momenta and elevation: the lagged depth is taken
+    // from the old stage where it is needed, max_stage goes with the sweep and
+    // the bookkeeping runs beside the main kernels.
+    const bool plain = c.bc_kind == 0 && c.n_forcing == 0;
+    const bool side = plain && aux && aux->stream;
     nl::NLArgs<R> n;
     n.a = a;
     n.nsq = p.manning_sq;
-    const int64_t wplane = p.pitch * (int64_t)(p.ny + 1);
-    R *w = (R *)c.nl_work;
-    n.lag0 = w;
-    for (int k = 0; k < 4; k++) n.adv[k] = w + (1 + k) * wplane;
-    for (int k = 0; k < 4; k++) n.flx[k] = w + (5 + k) * wplane;
-    n.fw = (const R *)c.fw;
-    n.plane = p.pitch * (int64_t)p.ny;
-    const dim3 block(32, 8), g1((p.nx + 31) / 32, (p.ny + 7) / 8), g2((p.nx + 32) / 32, (p.ny + 8) / 8);
+    n.lag0 = plain ? nullptr : (R *)c.nl_work;
+    n.chezy = c.chezy;
+    const dim3 block(32, 8), g1((p.nx + 31) / 32, (p.ny + 7) / 8);
+    const dim3 g2((p.nx + nl::TX - 1) / nl::TX, (p.ny + nl::TY - 1) / nl::TY);
     auto run = [&](int cat, auto &&launch) {
         hook(cat, 0);
         launch();
         hook(cat, 1);
     };
-    run(CAT_LINEAR_EDGE, [&] { nl::lag0_kernel<R><<<g1, block, 0, s>>>(n); });
-    run(CAT_LINEAR_EDGE, [&] { linear_edge_kernel<R><<<1, 512, 0, s>>>(a, sc, c.exterior_cells_width, c.bf); });
-    run(CAT_LINEAR_MAIN, [&] { nl::stage_kernel<R><<<g1, block, 0, s>>>(n); });
+    if (!plain) run(CAT_LINEAR_EDGE, [&] { nl::lag0_kernel<R><<<g1, block, 0, s>>>(n); });
+    cudaStream_t es = s;
+    if (side) {
+        es = aux->stream;
+        cudaEventRecord(aux->fork, s);
+        cudaStreamWaitEvent(es, aux->fork, 0);
+    }
+    run(CAT_LINEAR_EDGE, [&] { linear_edge_kernel<R><<<1, 512, 0, es>>>(a, sc, c.exterior_cells_width, c.bf); });
+    if (side) cudaEventRecord(aux->join, es);
+    run(CAT_LINEAR_MAIN, [&] {
+        nl::stage_kernel<R><<<g1, block, 0, s>>>(n, plain ? p.max_stage : nullptr, c.xl, c.xu, c.yl, c.yu);
+    });
     if (c.bc_kind == 3)   // flather_boundary
         run(CAT_LINEAR_EDGE, [&] {
             launch_leapfrog_boundary<R>(p.nx, p.ny, p.pitch, p.stg_o, const_cast<R *>(p.uh), const_cast<R *>(p.vh),
@@ -2317,26 +2365,16 @@ cudaError_t launch_leapfrog_nonlinear_step(const StepPlanes<R> &p, const Metrics
         launch_forcing<R>(c, clk, p.pitch, p.stg_o, const_cast<R *>(p.uh), const_cast<R *>(p.vh), p.elv, sc, s,
                           hook, CAT_LINEAR_EDGE);
     }
-    run(CAT_LINEAR_EDGE, [&] {
-        if (c.chezy)
-            friction_work_kernel<R, true><<<g1, block, 0, s>>>(a, p.manning_sq, (R *)c.fw, 0, 1, 0, p.nx - 1, 0,
-                                                               p.ny - 1);
-        else
-            friction_work_kernel<R, false><<<g1, block, 0, s>>>(a, p.manning_sq, (R *)c.fw, 0, 1, 0, p.nx - 1, 0,
-                                                                p.ny - 1);
-    });
-    run(CAT_LINEAR_MAIN, [&] { nl::advection_kernel<R><<<g1, block, 0, s>>>(n); });
-    run(CAT_LINEAR_MAIN, [&] { nl::flux_kernel<R><<<g2, block, 0, s>>>(n); });
     run(CAT_LINEAR_MAIN, [&] {
-        if (c.spherical && c.coriolis) nl::momentum_kernel<R, true, true><<<g1, block, 0, s>>>(n);
-        else if (c.spherical) nl::momentum_kernel<R, true, false><<<g1, block, 0, s>>>(n);
-        else nl::momentum_kernel<R, false, false><<<g1, block, 0, s>>>(n);
+        if (c.spherical && c.coriolis) nl::momentum_kernel<R, true, true><<<g2, nl::NT, 0, s>>>(n);
+        else if (c.spherical) nl::momentum_kernel<R, true, false><<<g2, nl::NT, 0, s>>>(n);
+        else nl::momentum_kernel<R, false, false><<<g2, nl::NT, 0, s>>>(n);
     });
-    run(CAT_LINEAR_MAIN, [&] { nl::dry_outflow_kernel<R><<<g1, block, 0, s>>>(n); });
-    if (p.max_stage)
+    if (p.max_stage && !plain)
         run(CAT_MAXSTAGE, [&] {
             launch_update_max_stage<R>(p.nx, p.ny, p.pitch, p.stg_o, p.max_stage, c, s);
         });
+    if (side) cudaStreamWaitEvent(s, aux->join, 0);
     return cudaGetLastError();
 }
 
@@ -2555,10 +2593,10 @@ cudaError_t launch_gauges(int64_t pitch, const R *stg, const R *uh, const R *vh,
 
 template cudaError_t launch_leapfrog_nonlinear_step<double>(const StepPlanes<double> &, const Metrics<double> &,
                                                              const StepConfig &, double, DevScalars *, cudaStream_t,
-                                                             const LaunchHook &);
+                                                             const LaunchHook &, const AuxStream *);
 template cudaError_t launch_leapfrog_nonlinear_step<float>(const StepPlanes<float> &, const Metrics<float> &,
                                                             const StepConfig &, float, DevScalars *, cudaStream_t,
-                                                            const LaunchHook &);
+                                                            const LaunchHook &, const AuxStream *);
 template cudaError_t launch_linear_step<double>(const StepPlanes<double> &, const Metrics<double> &,
                                                 const StepConfig &, double, DevScalars *, cudaStream_t,
                                                 const LaunchHook &, const AuxStream *);

@@ -63,19 +63,6 @@ template <typename R> struct RowConst {
     R cs, cu, cv, dxb, dxb1, dtc, dtj;   // dt/area, g dt/area, g dt/mean area, distance_bottom_edge(r), (r+1), dt cor/2 ...
 };
 
-// The semi-implicit friction multiplier 1 / ((1 + lf) + dt fw sqrt(m0^2 + mt^2)).
-__device__ __forceinline__ double friction_multiplier(double lf1, double dt, double fw, double m0, double mt)
-{
-    const double x = m0 * m0 + mt * mt;
-    const double d = lf1 + dt * fw * sqrt_ord(x);
-    if (x < 1.0e280 && d < 1.0e280) return rcp_ord(d);
-    return 1.0 / (lf1 + dt * fw * sqrt(x));   // a run that has blown up
-}
-__device__ __forceinline__ float friction_multiplier(float lf1, float dt, float fw, float m0, float mt)
-{
-    return 1.0f / (lf1 + dt * fw * sqrtf(m0 * m0 + mt * mt));
-}
-
 template <typename R, bool COR, bool TL, bool NLF, bool GAUGES>
 __global__ void __launch_bounds__(32 * WPC, pair_ctas(NLF, (int)sizeof(R))) linear_pair_kernel(const LinearPair<R> a, int SH, int nstrips)
 {

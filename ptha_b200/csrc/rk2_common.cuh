@@ -62,10 +62,6 @@ __device__ __forceinline__ void atomic_max_pos_double(unsigned long long *addr, 
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// 1 / depth of a wet cell.
-__device__ __forceinline__ double depth_inverse(double dep) { return dep < 1.0e280 ? rcp_ord(dep) : 1.0 / dep; }
-__device__ __forceinline__ float depth_inverse(float dep) { return 1.0f / dep; }
-
 // Whether a and b have the same sign bit.
 __device__ __forceinline__ bool same_sign(double a, double b) { return (__double2hiint(a) ^ __double2hiint(b)) >= 0; }
 __device__ __forceinline__ bool same_sign(float a, float b) { return (__float_as_int(a) ^ __float_as_int(b)) >= 0; }

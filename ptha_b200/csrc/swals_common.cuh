@@ -91,6 +91,23 @@ __device__ __forceinline__ double sqrt_ord(double x)
 }
 __device__ __forceinline__ float sqrt_ord(float x) { return sqrtf(x); }
 
+// 1 / depth of a wet cell.
+__device__ __forceinline__ double depth_inverse(double dep) { return dep < 1.0e280 ? rcp_ord(dep) : 1.0 / dep; }
+__device__ __forceinline__ float depth_inverse(float dep) { return 1.0f / dep; }
+
+// The semi-implicit friction multiplier 1 / ((1 + lf) + dt fw sqrt(m0^2 + mt^2)).
+__device__ __forceinline__ double friction_multiplier(double lf1, double dt, double fw, double m0, double mt)
+{
+    const double x = m0 * m0 + mt * mt;
+    const double d = lf1 + dt * fw * sqrt_ord(x);
+    if (x < 1.0e280 && d < 1.0e280) return rcp_ord(d);
+    return 1.0 / (lf1 + dt * fw * sqrt(x));   // a run that has blown up
+}
+__device__ __forceinline__ float friction_multiplier(float lf1, float dt, float fw, float m0, float mt)
+{
+    return 1.0f / (lf1 + dt * fw * sqrtf(m0 * m0 + mt * mt));
+}
+
 // Friction power law pow(x, p), p = fl(-7/3) (Manning) or -2 (Chezy), for
 // x >= minimum_allowed_depth (update_U_DE1_inner_include.f90:72-75).  The
 // oracle evaluates the same operation sequence, so both give the same bits

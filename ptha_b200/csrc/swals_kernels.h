@@ -81,7 +81,7 @@ struct StepConfig {
     void *ring;             // linear + Flather: 2 (nx + ny - 2) x 2 reals of ring momenta
     void *fw;               // leapfrog_linear_plus_nonlinear_friction: friction_work (2 planes), else null
     int fw_ready;           // truely linear: friction_work already computed (friction_work_is_setup)
-    void *nl_work;          // leapfrog_nonlinear: 9 work planes of pitch x (ny + 1)
+    void *nl_work;          // leapfrog_nonlinear: one work plane of pitch x (ny + 1)
     int n_forcing;          // forcing patches, applied in order (apply_forcing_patch_array)
     const ForcingPatch *forcing;
     void *eddy_visc;        // use_eddy_viscosity: one plane of per-cell eddy viscosity, else null
@@ -150,7 +150,8 @@ cudaError_t launch_leapfrog_boundary(int nx, int ny, int64_t pitch, R *stg, R *u
                                      const StepConfig &c, R dt, DevScalars *sc, cudaStream_t s);
 template <typename R>
 cudaError_t launch_leapfrog_nonlinear_step(const StepPlanes<R> &p, const Metrics<R> &m, const StepConfig &c, R dt,
-                                           DevScalars *sc, cudaStream_t s, const LaunchHook &hook);
+                                           DevScalars *sc, cudaStream_t s, const LaunchHook &hook,
+                                           const AuxStream *aux = nullptr);
 
 // The leapfrog's interior update alone (no boundary routine, boundary-flux
 // sums, time or max_stage): the linear map x' = M x that the adjoint
