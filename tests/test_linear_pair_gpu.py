@@ -85,3 +85,15 @@ def test_any_segment_height(rows, monkeypatch):
     a, b = (_run(kw, U, 5, (20,), pairs) for pairs in (True, False))
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["plain", "coriolis", "wet_faces_coriolis", "region"])
+@pytest.mark.parametrize("real_bytes", [8, 4])
+@pytest.mark.parametrize("rows", [1, 2, 7, 33])
+def test_segments_away_from_the_sides(rows, name, real_bytes, monkeypatch):
+    """Strips and segments with and without a side next to one another."""
+    monkeypatch.setenv("SWALS_PAIR_ROWS", str(rows))
+    kw, U = _case(430, 90, VARIANTS[name], real_bytes)
+    a, b = (_run(kw, U, 5, (10,), pairs) for pairs in (True, False))
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
