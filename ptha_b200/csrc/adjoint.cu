@@ -11,7 +11,9 @@
 // tile, the momentum-transpose contributions, forms the total stage adjoint
 // on the tile plus an east/north halo, then applies the stage transpose.
 // Reads lambda' (3 planes) and ELV, writes lambda (3 planes): the same 56 B
-// per cell (FP64) as a forward step.
+// per cell (FP64) as a forward step.  Sweeps take two steps a pass
+// (adjoint_pair.cu); the kernels here do an odd last step and planes that pass
+// cannot take.
 //
 // The reference has no adjoint; its correctness is checked by the
 // dot-product identity <M d, l> = <d, M^T l>, by central finite differences
@@ -329,22 +331,21 @@ __global__ void inject_kernel(R *ls, int64_t P, const int *site_ij, int n, const
     }
 }
 
-// Kernel choice: streaming unless SWALS_ADJOINT_KERNEL=tile.
-bool adjoint_tile()
+// Kernel choice (SWALS_ADJOINT_KERNEL): 1 single steps by the tile kernel, 2 by
+// the streaming kernel, 0 (unset, "pair") two steps a pass where the planes
+// allow it and the streaming kernel for the rest.
+int adjoint_kernel()
 {
     static int t = -1;
     if (t < 0) {
         const char *e = getenv("SWALS_ADJOINT_KERNEL");
-        t = (e && strcmp(e, "tile") == 0) ? 1 : 0;
+        t = !e || !*e || strcmp(e, "pair") == 0 ? 0 : strcmp(e, "tile") == 0 ? 1 : 2;
     }
-    return t == 1;
+    return t;
 }
 
-// One adjoint step lambda_out = M^T (lambda_in + C^T resid): with `resid`
-// (n gauges at `sites`) the injection is fused into the streaming kernel.
 template <typename R>
-cudaError_t adjoint_step(swals_domain *d, R *const in[3], R *const out[3], double dt, const int *sites = nullptr,
-                         int ng = 0, const double *resid = nullptr)
+AdjArgs<R> adjoint_args(swals_domain *d, R *const in[3], R *const out[3], double dt)
 {
     AdjArgs<R> a;
     a.nx = d->nx; a.ny = d->ny; a.P = d->pitch;
@@ -357,8 +358,18 @@ cudaError_t adjoint_step(swals_domain *d, R *const in[3], R *const out[3], doubl
     a.msl = R(d->cfg.msl_linear);
     const R lfc = R(d->cfg.linear_friction_coeff);
     a.mult = (lfc != R(0)) ? (R(1) / (R(1) + a.dt * lfc)) : R(1);
+    return a;
+}
+
+// One adjoint step lambda_out = M^T (lambda_in + C^T resid): with `resid`
+// (n gauges at `sites`) the injection is fused into the streaming kernel.
+template <typename R>
+cudaError_t adjoint_step(swals_domain *d, R *const in[3], R *const out[3], double dt, const int *sites = nullptr,
+                         int ng = 0, const double *resid = nullptr)
+{
+    const AdjArgs<R> a = adjoint_args<R>(d, in, out, dt);
     swals::LaunchHook hook = swals::hook_of(d);
-    if (adjoint_tile()) {
+    if (adjoint_kernel() == 1) {
         if (resid && ng > 0) {
             inject_kernel<R><<<1, 32, 0, d->stream>>>(const_cast<R *>(in[0]), d->pitch, sites, ng, resid);
             d->launches++;
@@ -383,6 +394,46 @@ cudaError_t adjoint_step(swals_domain *d, R *const in[3], R *const out[3], doubl
         linear_adjoint_stream_kernel<R, false><<<gx, 128, 0, d->stream>>>(a, sh, nstrips, total, sites, ng, resid);
     hook(swals::CAT_LINEAR_MAIN, 1);
     return cudaGetLastError();
+}
+
+// `count` adjoint steps of lam[c], by pairs where the planes allow it, resid
+// (or null) count x ng residuals injected from the last; returns the buffer
+// they end in.  An even count ends where it began, as in map_steps.
+template <typename R>
+int adjoint_steps(swals_domain *d, R *const lam[2][3], int c, int count, double dt, const int *sites, int ng,
+                  const double *resid, cudaError_t &err)
+{
+    const swals::LaunchHook hook = swals::hook_of(d);
+    swals::StepPlanes<R> probe;
+    probe.nx = d->nx; probe.ny = d->ny; probe.pitch = d->pitch;
+    probe.stg = lam[0][0]; probe.uh = lam[0][1]; probe.vh = lam[0][2];
+    probe.stg_o = lam[1][0]; probe.uh_o = lam[1][1]; probe.vh_o = lam[1][2];
+    probe.elv = (R *)d->elv;
+    probe.max_stage = nullptr;
+    int pairs = adjoint_kernel() == 0 && swals::linear_pair_fits<R>(probe, 0, 0) ? count / 2 : 0;
+    if (count % 2 == 0 && pairs % 2 == 1) pairs--;
+    int n = count;
+    for (int k = 0; k < pairs && err == cudaSuccess; k++, n -= 2, c = 1 - c) {
+        const AdjArgs<R> s = adjoint_args<R>(d, lam[c], lam[1 - c], dt);
+        swals::AdjointPair<R> a;
+        a.nx = s.nx; a.ny = s.ny; a.P = s.P;
+        a.ls = s.ls; a.lu = s.lu; a.lv = s.lv;
+        a.ls_o = s.ls_o; a.lu_o = s.lu_o; a.lv_o = s.lv_o;
+        a.elv = s.elv; a.m = s.m;
+        a.xl = s.xl; a.xu = s.xu; a.yl = s.yl; a.yu = s.yu;
+        a.dt = s.dt; a.msl = s.msl; a.mult = s.mult;
+        a.sites = sites;
+        a.ng = resid ? ng : 0;
+        a.resid = resid ? resid + (size_t)(n - 1) * ng : nullptr;
+        a.resid2 = resid ? resid + (size_t)(n - 2) * ng : nullptr;
+        hook(swals::CAT_LINEAR_MAIN, 0);
+        err = swals::launch_adjoint_pair<R>(a, d->cfg.coriolis != 0, d->stream);
+        hook(swals::CAT_LINEAR_MAIN, 1);
+    }
+    for (; n > 0 && err == cudaSuccess; n--, c = 1 - c)
+        err = adjoint_step<R>(d, lam[c], lam[1 - c], dt, resid ? sites : nullptr, resid ? ng : 0,
+                              resid ? resid + (size_t)(n - 1) * ng : nullptr);
+    return c;
 }
 
 // The domain's adjoint scratch, grown to at least `need` bytes.
@@ -464,12 +515,9 @@ int adjoint_sweep(swals_domain *d, int nsteps, double dt, const double *gadj_hos
         void *dst[3] = {lam[0][0], lam[0][1], lam[0][2]};
         rc = copy_plane3(d, dst, (void *)lambda_seed_host, true);
     }
-    for (int n = nsteps; n >= 1 && rc == SWALS_OK; n--) {
-        const bool inj = ng > 0 && gadj_host;
-        e = adjoint_step<R>(d, lam[cur], lam[1 - cur], dt, inj ? d_sites : nullptr, inj ? ng : 0,
-                            inj ? d_g + (size_t)(n - 1) * ng : nullptr);
+    if (rc == SWALS_OK) {
+        cur = adjoint_steps<R>(d, lam, cur, nsteps, dt, d_sites, ng, ng > 0 && gadj_host ? d_g : nullptr, e);
         if (e != cudaSuccess) rc = swals::api_cuda_fail(e, "adjoint step");
-        cur = 1 - cur;
     }
     if (rc == SWALS_OK) {
         void *src[3] = {lam[cur][0], lam[cur][1], lam[cur][2]};
@@ -569,8 +617,8 @@ __global__ void loss_sum_kernel(const double *step_half, int n, double *loss)
 // then, for each segment from the last, the segment's forward steps are
 // recomputed from its checkpoint, recording the gauge stage, the segment's
 // residuals are formed, and the adjoint runs back through the segment with
-// the residuals injected as it goes.  Per timestep that is one forward map,
-// one recomputed forward map and one adjoint launch.  The recomputation of
+// the residuals injected as it goes.  Per two timesteps that is one forward
+// pass, one recomputed forward pass and one adjoint pass.  The recomputation of
 // segment s-1 does not depend on the adjoint through segment s, so it runs
 // on the domain's side stream, into a second buffer set, while the adjoint
 // runs on the main stream: the two grids are smaller than one wave of the
@@ -637,11 +685,9 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
         ck(err, "recompute");
     };
     auto adj_seq = [&](int count, int lc, int set) {   // adjoint back through `count` steps
-        for (int t = count; t > 0; t--) {
-            ck(adjoint_step<R>(d, lam[lc], lam[1 - lc], dt, d_sites, ng, d_resid[set] + (size_t)(t - 1) * ng),
-               "adjoint");
-            lc = 1 - lc;
-        }
+        cudaError_t err = cudaSuccess;
+        lc = adjoint_steps<R>(d, lam, lc, count, dt, d_sites, ng, d_resid[set], err);
+        ck(err, "adjoint");
         return lc;
     };
     const bool graphs = (K % 2 == 0) && K <= nsteps && !d->timers_on;

@@ -42,23 +42,15 @@
 #include <cstdlib>
 #include <type_traits>
 
-#include "swals_kernels.h"
+#include "pair_common.cuh"
 
 namespace swals {
 namespace {
 
+using pair::FULL;
+using pair::cp16;
+
 constexpr int SLOTS = 4;    // ring slots per warp: rows r - 1, r and two in flight
-constexpr unsigned FULL = 0xffffffffu;
-
-template <typename R> struct Vec;
-template <> struct Vec<double> { typedef double2 T; };
-template <> struct Vec<float> { typedef float4 T; };
-
-__device__ __forceinline__ void cp16(void *smem, const void *gmem, int src_bytes)
-{
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(src_bytes));
-}
 
 // Warps per SM that the register cap leaves room for (168 a thread for 12).
 // Fewer do not hide the latencies, more spill: 3600 x 2400 FP32 Coriolis 37.3
@@ -81,7 +73,7 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
     constexpr int OUTC = 30 * CPL;
     constexpr int NP = NLF ? 7 : 5;      // UH, VH, STG, ELV, max_stage and friction work at UH, VH of row r-1
     constexpr bool AVG = COR || NLF;     // the two-point averages of the other momentum
-    typedef typename Vec<R>::T V;
+    typedef typename pair::Vec<R>::T V;
     struct Face { R gu[CPL], gv[CPL], cu[CPL], cv[CPL], wi[CPL], wj[CPL]; };
     extern __shared__ __align__(16) unsigned char pair_smem[];
     RowConst<R> *rc = reinterpret_cast<RowConst<R> *>(pair_smem + sizeof(V) * 32 * NP * SLOTS);
@@ -136,11 +128,12 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
     }
     // gauges in this lane's own columns (up to 64 sites; more are looked up cell by cell)
     unsigned long long gm = 0ull;
-    if (GAUGES && out)
-        for (int q = 0; q < min(a.g_n, 64); q++)
-            if (a.g_sites[2 * q] >= c0 && a.g_sites[2 * q] < c0 + CPL && a.g_sites[2 * q + 1] >= ra &&
-                a.g_sites[2 * q + 1] < rb)
-                gm |= 1ull << q;
+    if (GAUGES)
+        for (unsigned long long m = pair::sites_in(a.g_sites, a.g_n, strip * OUTC, strip * OUTC + OUTC - 1, ra, rb - 1, lane); m;
+             m &= m - 1) {
+            const int q = __ffsll((long long)m) - 1;
+            if (out && a.g_sites[2 * q] >= c0 && a.g_sites[2 * q] < c0 + CPL) gm |= 1ull << q;
+        }
     auto record = [&](int step, int row, const R(&s)[CPL], const R(&u)[CPL], const R(&v)[CPL]) {
         if (rec + step >= a.g_capacity) return;
         auto put = [&](int q) {
@@ -504,6 +497,26 @@ __global__ void __launch_bounds__(512) linear_pair_edge_kernel(const LinearPair<
     }
 }
 
+template <typename R, bool COR, bool TL, bool NLF>
+cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
+{
+    constexpr int CPL = 16 / (int)sizeof(R);
+    const int nstrips = (a.p.nx + 30 * CPL - 1) / (30 * CPL);
+    const int sh = pair::rows((int64_t)nstrips * a.nbatch, a.p.ny, pair_warps(NLF, (int)sizeof(R)), NLF);
+    const int64_t ctas = (int64_t)nstrips * ((a.p.ny + sh - 1) / sh) * a.nbatch;
+    const size_t smem = 16 * 32 * (NLF ? 7 : 5) * SLOTS + sizeof(RowConst<R>) * (sh + 4);
+    auto go = [&](auto kernel) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        if (e != cudaSuccess) return e;
+        kernel<<<(unsigned)ctas, 32, smem, s>>>(a, sh, nstrips);
+        return cudaGetLastError();
+    };
+    if (a.g_n > 0) return go(linear_pair_kernel<R, COR, TL, NLF, true>);
+    return go(linear_pair_kernel<R, COR, TL, NLF, false>);
+}
+
+}  // namespace
+
 // Rows per segment (SWALS_PAIR_ROWS sets it): the count with the least
 // estimate, over the rounds in which an SM takes its `resident` warps, of
 //   (rows + 4) x sum of (A + warps of the round / 4),
@@ -517,7 +530,7 @@ __global__ void __launch_bounds__(512) linear_pair_edge_kernel(const LinearPair<
 // 32 34.4.  Beyond three rounds the HBM binds and 16 rows keep the rows that
 // neighbours share in L2: 4096^2 FP32 14 59.7, 28 62.3, 64 70.1; FP64 16 112.1,
 // 42 114.4, 85 120.0.
-int pair_rows(int64_t strips, int ny, int resident, bool friction)
+int pair::rows(int64_t strips, int ny, int resident, bool friction)
 {
     const char *e = getenv("SWALS_PAIR_ROWS");
     if (e && atoi(e) > 0) return std::min(atoi(e), 256);
@@ -543,26 +556,6 @@ int pair_rows(int64_t strips, int ny, int resident, bool friction)
     }
     return best;
 }
-
-template <typename R, bool COR, bool TL, bool NLF>
-cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
-{
-    constexpr int CPL = 16 / (int)sizeof(R);
-    const int nstrips = (a.p.nx + 30 * CPL - 1) / (30 * CPL);
-    const int sh = pair_rows((int64_t)nstrips * a.nbatch, a.p.ny, pair_warps(NLF, (int)sizeof(R)), NLF);
-    const int64_t ctas = (int64_t)nstrips * ((a.p.ny + sh - 1) / sh) * a.nbatch;
-    const size_t smem = 16 * 32 * (NLF ? 7 : 5) * SLOTS + sizeof(RowConst<R>) * (sh + 4);
-    auto go = [&](auto kernel) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)ctas, 32, smem, s>>>(a, sh, nstrips);
-        return cudaGetLastError();
-    };
-    if (a.g_n > 0) return go(linear_pair_kernel<R, COR, TL, NLF, true>);
-    return go(linear_pair_kernel<R, COR, TL, NLF, false>);
-}
-
-}  // namespace
 
 template <typename R>
 bool linear_pair_fits(const StepPlanes<R> &p, int64_t inst_stride, int64_t max_stride)

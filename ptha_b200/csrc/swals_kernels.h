@@ -196,6 +196,26 @@ cudaError_t launch_linear_pair(LinearPair<R> a, const StepConfig &c, cudaStream_
 template <typename R>
 cudaError_t launch_linear_pair_edge(const LinearPair<R> &a, const StepConfig &c, DevScalars *sc, cudaStream_t s);
 
+// Two adjoint steps of the truly linear leapfrog in one pass (adjoint_pair.cu):
+// lambda_o = M^T (C^T resid2 + M^T (C^T resid + lambda)), for planes that
+// linear_pair_fits accepts.
+template <typename R>
+struct AdjointPair {
+    int nx, ny;
+    int64_t P;
+    const R *ls, *lu, *lv;   // adjoint of the later step's outputs
+    R *ls_o, *lu_o, *lv_o;   // adjoint of the earlier step's inputs
+    const R *elv;
+    Metrics<R> m;
+    int xl, xu, yl, yu;
+    R dt, msl, mult;         // mult: linear friction factor (1 without friction)
+    const int *sites;        // ng gauge cells (i, j); ng = 0: none
+    int ng;
+    const double *resid, *resid2;
+};
+template <typename R>
+cudaError_t launch_adjoint_pair(const AdjointPair<R> &a, bool coriolis, cudaStream_t s);
+
 // Batched truly/not-truly linear leapfrog: `nbatch` instances whose planes
 // follow instance 0's at `inst_stride` elements, sharing ELV and metrics
 // (no boundary routine).  tile_cfg selects one of linear_tile_config_count()
