@@ -16,6 +16,7 @@
 //     and the lines that only the update reads are started towards L2.
 #include "rk2_common.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -301,22 +302,22 @@ __global__ void __launch_bounds__(SW, strip_min_ctas(MODE, EDDY, (int)sizeof(R))
 // CTAs of a launch with sh rows per strip segment.
 int64_t fv_ctas(int nx, int ny, int sh) { return (int64_t)((nx + SO - 1) / SO) * ((ny + sh - 1) / sh); }
 
-// Rows per strip segment for a grid (SWALS_FV_ROWS sets it): the candidate
-// with the least estimate of the time a segment's CTAs take,
-//   (rows + 2) x CTA-rows that an SM works through per row of a segment.
-// The two rows stand for the lead-in, whose rows do part of a row's work.  An
-// SM runs up to five CTAs side by side; fewer than three take the time of
-// three (a row of one CTA is a serial chain: 2.6 us a row for one pass at
-// 300 x 200, against 0.76 us a CTA-row on full SMs); CTAs beyond the five
-// follow as others end, which hides most of a last, smaller round.
-// Measured on the B200, a step in us, the estimate's rows against the best
-// of 1 .. 32 and the 8 or 12 taken before: rk2 FP64 120 x 80 1 row 32.0
-// (8 rows 71.0), 300 x 200 2: 42.6 (8: 71.0), 520 x 390 5: 66.1 (4: 65.0,
-// 8: 78.0), 930^2 14: 160.3 (5: 156.4, 8: 172.0), 1275 x 879 14: 198.1
-// (7: 192.4, 12: 216.2), 2048^2 16: 556.5 (12: 557.9); midpoint 930^2 14:
-// 144.2 (8: 152.5).  Over 20 grids, methods and both precisions 1.4 % above
-// the best on average, 5.5 % at most.
-int fv_rows(int nx, int ny)
+// Rows per strip segment for a grid (SWALS_FV_ROWS sets it): the count with
+// the least estimate, over the rounds in which an SM takes its `resident`
+// CTAs, of
+//   (rows + 1.5) x sum of (2, or 0.75 after the first round, + CTAs of the round).
+// The 1.5 rows stand for the lead-in, whose rows do part of a row's work; the
+// 2 for the chain of a row, that few CTAs leave bare and that the CTAs of a
+// later round mostly start under.  `resident` is the kernel's own: a round of
+// four is full where one of five would not be.  Measured on the B200, us a
+// launch, the estimate's rows (best of 1 .. 32): flux kernel FP64 300 x 200 2
+// 15.2, 600 x 500 6 28.5, 930^2 13 57.8, 1275 x 879 6 72.6 (10: 72.5), 2048^2
+// 20 209.5 (16: 207.6), FP32 1531 x 1021 7 73.7 (9: 72.1); stage 2 1 16.7, 6
+// 33.1, 13 70.4 (5: 69.9), 7 86.7, 16 252.9, 7 90.5 (9: 88.4); midpoint's two
+// stages 930^2 13 137.0, 500 x 700 6 74.2: 0.5 % above the best on average, 2.4
+// at most.  One line for all kernels over fewer counts had taken 145.1 and
+// 80.0 for the last two, 79.9 for the flux kernel at 1275 x 879.
+int fv_rows(int nx, int ny, int resident)
 {
     const char *e = getenv("SWALS_FV_ROWS");
     if (e && atoi(e) > 0) return atoi(e);
@@ -326,20 +327,13 @@ int fv_rows(int nx, int ny)
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         sms = n;
     }
-    const int cand[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16};
-    constexpr double resident = 5.0, chain = 3.0, exposed = 0.3;
     int best = 0;
     double best_cost = 0.0;
-    for (int sh : cand) {
-        const double ctas = (double)fv_ctas(nx, ny, sh) / sms;
-        double w;
-        if (ctas <= resident) {
-            w = std::fmax(chain, std::ceil(ctas));
-        } else {
-            const double rest = std::fmod(ctas, resident);
-            w = ctas + (rest > 0.0 ? exposed * std::fmax(chain - rest, 0.0) : 0.0);
-        }
-        const double cost = (sh + 2.0) * w;
+    for (int sh = 1; sh <= 32; sh++) {
+        double t = 0.0, chain = 2.0;
+        for (double left = (double)fv_ctas(nx, ny, sh) / sms; left > 1e-9; left -= resident, chain = 0.75)
+            t += chain + std::min(std::ceil(left), (double)resident);
+        const double cost = (sh + 1.5) * t;
         if (best == 0 || cost < best_cost) {
             best = sh;
             best_cost = cost;
@@ -356,10 +350,11 @@ cudaError_t launch_stage_stream(const Rk2Args<R> &a, cudaStream_t s)
     // Stage 2 takes the first stage's dt and accumulates no CFL maximum: its
     // kernels leave the edges' wave-speed candidates out.
     if (MODE == MODE_STAGE2 && a.write_cfl) return cudaErrorInvalidValue;
-    const int SH = fv_rows(a.nx, a.ny);
+    const bool eddy = MODE != MODE_CFL && (a.flux_variant & FLUX_EDDY);
+    const int SH = fv_rows(a.nx, a.ny, strip_min_ctas(MODE, eddy, (int)sizeof(R)));
     const int blocks = (int)fv_ctas(a.nx, a.ny, SH);
     if constexpr (MODE != MODE_CFL) {
-        if (a.flux_variant & FLUX_EDDY) {
+        if (eddy) {
             rk2_strip_kernel<R, MODE, SPH, COR, FRIC, true><<<blocks, SW, 0, s>>>(a, SH);
             return cudaGetLastError();
         }
