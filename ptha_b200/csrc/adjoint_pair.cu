@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(32, RESIDENT) adjoint_pair_kernel(const Adjoin
         rc[k] = c;
     }
     __syncwarp();
+    after_previous();   // (the metrics above are no kernel's output)
+    let_next_start();
 
     const int c0 = strip * OUTC + (lane - 1) * CPL;          // this lane's first column
     const bool out = lane >= 1 && lane <= 30 && c0 < nx;
@@ -322,9 +324,8 @@ cudaError_t launch_adjoint_pair(const AdjointPair<R> &a, bool coriolis, cudaStre
     const int sh = pair::rows(nstrips, a.ny, RESIDENT, false);
     const unsigned ctas = (unsigned)(nstrips * ((a.ny + sh - 1) / sh));
     const size_t smem = 16 * (32 * NP + 1) * SLOTS + sizeof(RowConst<R>) * (sh + 4);
-    if (coriolis) adjoint_pair_kernel<R, true><<<ctas, 32, smem, s>>>(a, sh, nstrips);
-    else adjoint_pair_kernel<R, false><<<ctas, 32, smem, s>>>(a, sh, nstrips);
-    return cudaGetLastError();
+    if (coriolis) return launch_behind(adjoint_pair_kernel<R, true>, ctas, 32, smem, s, a, sh, nstrips);
+    return launch_behind(adjoint_pair_kernel<R, false>, ctas, 32, smem, s, a, sh, nstrips);
 }
 template cudaError_t launch_adjoint_pair<double>(const AdjointPair<double> &, bool, cudaStream_t);
 template cudaError_t launch_adjoint_pair<float>(const AdjointPair<float> &, bool, cudaStream_t);

@@ -2139,6 +2139,7 @@ __device__ __forceinline__ Adv<R> advection(const NLArgs<R> &n, int i, int r, La
 template <typename R, bool SPH, bool COR>
 __global__ void __launch_bounds__(NT, 5) momentum_kernel(NLArgs<R> n)
 {
+    after_previous();
     const LinArgs<R> &a = n.a;
     const int nx = a.p.nx, ny = a.p.ny;
     const int64_t P = a.p.pitch;
@@ -2366,9 +2367,9 @@ cudaError_t launch_leapfrog_nonlinear_step(const StepPlanes<R> &p, const Metrics
                           hook, CAT_LINEAR_EDGE);
     }
     run(CAT_LINEAR_MAIN, [&] {
-        if (c.spherical && c.coriolis) nl::momentum_kernel<R, true, true><<<g2, nl::NT, 0, s>>>(n);
-        else if (c.spherical) nl::momentum_kernel<R, true, false><<<g2, nl::NT, 0, s>>>(n);
-        else nl::momentum_kernel<R, false, false><<<g2, nl::NT, 0, s>>>(n);
+        if (c.spherical && c.coriolis) launch_behind(nl::momentum_kernel<R, true, true>, g2, nl::NT, 0, s, n);
+        else if (c.spherical) launch_behind(nl::momentum_kernel<R, true, false>, g2, nl::NT, 0, s, n);
+        else launch_behind(nl::momentum_kernel<R, false, false>, g2, nl::NT, 0, s, n);
     });
     if (p.max_stage && !plain)
         run(CAT_MAXSTAGE, [&] {

@@ -103,6 +103,8 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
         rc[k] = c;
     }
     __syncthreads();
+    after_previous();   // (the metrics above are no kernel's output)
+    let_next_start();
     const int rec = GAUGES ? (a.g_count ? *a.g_count : 0) : 0;
 
     const int64_t io = (int64_t)b * a.inst_stride;
@@ -508,8 +510,7 @@ cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
     auto go = [&](auto kernel) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)ctas, 32, smem, s>>>(a, sh, nstrips);
-        return cudaGetLastError();
+        return launch_behind(kernel, (unsigned)ctas, 32, smem, s, a, sh, nstrips);
     };
     if (a.g_n > 0) return go(linear_pair_kernel<R, COR, TL, NLF, true>);
     return go(linear_pair_kernel<R, COR, TL, NLF, false>);

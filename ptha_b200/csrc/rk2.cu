@@ -326,6 +326,7 @@ __device__ __forceinline__ RingVal<R> we_value(const BcArgs<R> &a, int i, int r,
 template <typename R, int KIND>
 __global__ void __launch_bounds__(256) rk2_boundary_kernel(const BcArgs<R> a)
 {
+    after_previous();
     const int nx = a.nx, ny = a.ny;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     // Ring cells, each once: rows 0 and ny-1 in full, then columns 0 and
@@ -413,10 +414,9 @@ cudaError_t launch_boundary(const BcArgs<R> &b, cudaStream_t s)
 {
     const int n = 2 * b.nx + 2 * (b.ny - 2);
     const int blocks = (n + 255) / 256;
-    if (b.kind == 1) rk2_boundary_kernel<R, 1><<<blocks, 256, 0, s>>>(b);
-    else if (b.kind == 3) rk2_boundary_kernel<R, 3><<<blocks, 256, 0, s>>>(b);
-    else rk2_boundary_kernel<R, 2><<<blocks, 256, 0, s>>>(b);
-    return cudaGetLastError();
+    if (b.kind == 1) return launch_behind(rk2_boundary_kernel<R, 1>, blocks, 256, 0, s, b);
+    if (b.kind == 3) return launch_behind(rk2_boundary_kernel<R, 3>, blocks, 256, 0, s, b);
+    return launch_behind(rk2_boundary_kernel<R, 2>, blocks, 256, 0, s, b);
 }
 
 // End of a step: domain%max_dt, time, boundary-flux integrals, counters
@@ -461,6 +461,7 @@ __global__ void __launch_bounds__(1024) rk2_finalize_kernel(int nx, int ny, int 
                                                             int dt_from_cfl, double dt_fixed, double max_dt_inv_init,
                                                             DevScalars *sc, FinGauges<R> g)
 {
+    after_previous();
     constexpr int NSETS = (KIND == FIN_EULER) ? 1 : (KIND == FIN_RK2N) ? RK2N_N : 2;
     __shared__ double red[4 * NSETS][32];
     // gauges first: every read of the record count precedes thread 0's update
@@ -666,6 +667,7 @@ __device__ __forceinline__ void update_cell(const Rk2Args<R> &a, int i, int r, R
 template <typename R, bool SPH, bool COR, int FRIC>
 __global__ void __launch_bounds__(256, SWALS_UPDATE_MINB) rk2_update_kernel(const Rk2Args<R> a)
 {
+    after_previous();
     constexpr int NC = SWALS_UPDATE_CELLS;
     const int i0 = (blockIdx.x * 32 + threadIdx.x) * NC;
     const int r = blockIdx.y * 8 + threadIdx.y;
@@ -721,8 +723,7 @@ cudaError_t launch_update(const Rk2Args<R> &a, cudaStream_t s)
 {
     constexpr int NC = SWALS_UPDATE_CELLS;
     dim3 block(32, 8), grid((a.nx + 32 * NC - 1) / (32 * NC), (a.ny + 7) / 8);
-    rk2_update_kernel<R, SPH, COR, FRIC><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_behind(rk2_update_kernel<R, SPH, COR, FRIC>, grid, block, 0, s, a);
 }
 
 // Run F<R, SPH, COR, FRIC>(a, s) for the step configuration.
@@ -1063,7 +1064,7 @@ cudaError_t launch_rk2_step(R *const planes[3][3], int &cur, R *elv, R *max_stag
             if (e != cudaSuccess) return e;
         }
         hook(CAT_FINALIZE, 0);
-        rk2_finalize_kernel<R, FIN_EULER><<<1, 1024, 0, s>>>(nx, ny, c.exterior_cells_width, lines1,
+        e = launch_behind(rk2_finalize_kernel<R, FIN_EULER>, 1, 1024, 0, s, nx, ny, c.exterior_cells_width, lines1,
                                                              a.dt_from_cfl, dt, max_dt_inv_init, sc,
                                                              fin_gauges<R>(c, planes[B], pitch));
         hook(CAT_FINALIZE, 1);
@@ -1088,7 +1089,7 @@ cudaError_t launch_rk2_step(R *const planes[3][3], int &cur, R *elv, R *max_stag
             if (e != cudaSuccess) return e;
         }
         hook(CAT_FINALIZE, 0);
-        rk2_finalize_kernel<R, FIN_RK2><<<1, 1024, 0, s>>>(nx, ny, c.exterior_cells_width, lines1, a.dt_from_cfl,
+        e = launch_behind(rk2_finalize_kernel<R, FIN_RK2>, 1, 1024, 0, s, nx, ny, c.exterior_cells_width, lines1, a.dt_from_cfl,
                                                            dt, max_dt_inv_init, sc,
                                                            fin_gauges<R>(c, planes[C], pitch));
         hook(CAT_FINALIZE, 1);
@@ -1120,7 +1121,7 @@ cudaError_t launch_rk2_step(R *const planes[3][3], int &cur, R *elv, R *max_stag
         if (e != cudaSuccess) return e;
     }
     hook(CAT_FINALIZE, 0);
-    rk2_finalize_kernel<R, FIN_RK2><<<1, 1024, 0, s>>>(nx, ny, c.exterior_cells_width, lines1, a.dt_from_cfl,
+    e = launch_behind(rk2_finalize_kernel<R, FIN_RK2>, 1, 1024, 0, s, nx, ny, c.exterior_cells_width, lines1, a.dt_from_cfl,
                                               dt, max_dt_inv_init, sc, fin_gauges<R>(c, planes[C], pitch));
     hook(CAT_FINALIZE, 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1199,7 +1200,7 @@ cudaError_t launch_midpoint_step(R *const planes[3][3], int &cur, R *elv, R *max
         if (e != cudaSuccess) return e;
     }
     hook(CAT_FINALIZE, 0);
-    rk2_finalize_kernel<R, FIN_MIDPOINT><<<1, 1024, 0, s>>>(nx, ny, c.exterior_cells_width, lines1,
+    e = launch_behind(rk2_finalize_kernel<R, FIN_MIDPOINT>, 1, 1024, 0, s, nx, ny, c.exterior_cells_width, lines1,
                                                             has_dt ? 0 : 1, dt, a.max_dt_inv_init, sc,
                                                             fin_gauges<R>(c, planes[C], pitch));
     hook(CAT_FINALIZE, 1);
@@ -1261,7 +1262,7 @@ cudaError_t launch_rk2n_step(R *const planes[3][3], int &cur, R *elv, R *max_sta
     hook(CAT_MAXSTAGE, 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     hook(CAT_FINALIZE, 0);
-    rk2_finalize_kernel<R, FIN_RK2N><<<1, 1024, 0, s>>>(nx, ny, c.exterior_cells_width, lines, has_dt ? 0 : 1,
+    e = launch_behind(rk2_finalize_kernel<R, FIN_RK2N>, 1, 1024, 0, s, nx, ny, c.exterior_cells_width, lines, has_dt ? 0 : 1,
                                               dt_sub, a.max_dt_inv_init, sc, fin_gauges<R>(c, planes[U5], pitch));
     hook(CAT_FINALIZE, 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

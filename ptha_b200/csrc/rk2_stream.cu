@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(SW, strip_min_ctas(MODE, EDDY, (int)sizeof(R))
 {
     constexpr bool UPDATE = (MODE == MODE_STAGE1 || MODE == MODE_STAGE2);
     __shared__ Strip<R> sm;
+    after_previous();
     const int lane = threadIdx.x, l = lane + 1;
     const int nx = a.nx, ny = a.ny;
     const int strips_x = (nx + SO - 1) / SO;
@@ -355,12 +356,10 @@ cudaError_t launch_stage_stream(const Rk2Args<R> &a, cudaStream_t s)
     const int blocks = (int)fv_ctas(a.nx, a.ny, SH);
     if constexpr (MODE != MODE_CFL) {
         if (eddy) {
-            rk2_strip_kernel<R, MODE, SPH, COR, FRIC, true><<<blocks, SW, 0, s>>>(a, SH);
-            return cudaGetLastError();
+            return launch_behind(rk2_strip_kernel<R, MODE, SPH, COR, FRIC, true>, blocks, SW, 0, s, a, SH);
         }
     }
-    rk2_strip_kernel<R, MODE, SPH, COR, FRIC, false><<<blocks, SW, 0, s>>>(a, SH);
-    return cudaGetLastError();
+    return launch_behind(rk2_strip_kernel<R, MODE, SPH, COR, FRIC, false>, blocks, SW, 0, s, a, SH);
 }
 
 #define SWALS_INST(R, MODE, SPH, COR, FRIC) \

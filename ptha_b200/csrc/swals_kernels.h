@@ -24,6 +24,40 @@ struct LaunchHook {
     void operator()(int cat, int phase) const { if (fn) fn(ctx, cat, phase); }
 };
 
+// Launch of a kernel that may start while the launch before it on the stream
+// still ends: it must call after_previous() before it touches what that one
+// reads or writes.  Hides the launch and the prologue behind the tail.
+// Measured: 15 rk2 steps of 300 x 200 called one by one 798 -> 588 us, rk2 120 x
+// 80 in a graph 32.9 -> 30.6 us a step, adjoint pairs 400^2 5.2 -> 3.9 and 1200
+// x 800 12.0 -> 10.7, linear pairs 400^2 5.3 -> 4.9; nothing on grids whose
+// passes take 100 us.
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Lets the launch behind this one take its places as this one's CTAs leave
+// them, for kernels with a prologue of their own before after_previous(); the
+// finite-volume kernels, without one, are up to 3 % slower with it.
+__device__ __forceinline__ void let_next_start()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename R>
 struct StepPlanes {
     int nx, ny;
