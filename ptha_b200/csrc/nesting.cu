@@ -617,6 +617,22 @@ struct swals_multidomain {
     std::vector<double> dx;   // all_dx_md: each domain's cell size as the setup computed it
     std::vector<Ex> ex;
     cudaStream_t stream = nullptr;
+    // The domains' sub-steps between two exchanges run side by side, domain k
+    // on branch k % BRANCHES, forked from and joined to `stream` every step:
+    // they share nothing in between, and their small kernels and last waves
+    // leave most of the chip idle (4 domains of 0.5 - 1.1 million cells, nine
+    // and ten sub-steps: 10.9 -> 8.9 ms for three steps).
+    static constexpr int BRANCHES = 8;
+    cudaStream_t branch[BRANCHES] = {};
+    cudaEvent_t fork = nullptr, joined[BRANCHES] = {};
+    void drop_branches()
+    {
+        for (cudaStream_t b : branch)
+            if (b) cudaStreamDestroy(b);
+        for (cudaEvent_t e : joined)
+            if (e) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+    }
     int device = 0;
     void *pool = nullptr;
     Ex *d_ex = nullptr;
@@ -787,18 +803,18 @@ int build_corrections(const swals_multidomain *md, int dj, const int32_t *pind, 
     return SWALS_OK;
 }
 
-static int integrals_scale(swals_multidomain *md, int k, double c)
+static int integrals_scale(swals_multidomain *md, int k, double c, cudaStream_t st)
 {
     // nesting_boundary_flux_integral_multiply: every send and recv box of domain k.
     for (const Ex &e : md->ex) {
         if (e.sdom == k) {
             const int64_t n = 4 * (2 * e.s_len[0] + 2 * e.s_len[2]);
-            scale_kernel<<<grid_for(n), 256, 0, md->stream>>>(md->d_int + e.s_int, n, c);
+            scale_kernel<<<grid_for(n), 256, 0, st>>>(md->d_int + e.s_int, n, c);
             md->launches++;
         }
         if (e.rdom == k) {
             const int64_t n = 4 * (2 * e.r_len[0] + 2 * e.r_len[2]);
-            scale_kernel<<<grid_for(n), 256, 0, md->stream>>>(md->d_int + e.r_int, n, c);
+            scale_kernel<<<grid_for(n), 256, 0, st>>>(md->d_int + e.r_int, n, c);
             md->launches++;
         }
     }
@@ -807,7 +823,7 @@ static int integrals_scale(swals_multidomain *md, int k, double c)
 }
 
 template <typename R>
-static int integral_step(swals_multidomain *md, int k, int phase, int A, double dt_local)
+static int integral_step(swals_multidomain *md, int k, int phase, int A, double dt_local, cudaStream_t st)
 {
     swals_domain *d = md->doms[k];
     const auto &pd = md->per[k];
@@ -816,14 +832,14 @@ static int integral_step(swals_multidomain *md, int k, int phase, int A, double 
     const Metrics<R> m = metrics_of<R>(d);
     if (is_linear_leapfrog(d->method)) {
         if (phase != 0) return SWALS_OK;
-        integral_leapfrog_kernel<R><<<grid_for(pd.nitems), 256, 0, md->stream>>>(
+        integral_leapfrog_kernel<R><<<grid_for(pd.nitems), 256, 0, st>>>(
             p, m.dxb, m.dyl, pd.d_box, pd.nbox, pd.nitems, md->d_int, R(dt_local));
     } else {
         if (phase != 1) return SWALS_OK;
         const int B = (A + 1) % 3;
         const bool euler = (d->method == M_EULER);
         const R dts = euler ? R(dt_local) : R(R(dt_local) * R(0.5));
-        integral_fv_kernel<R><<<grid_for(pd.nitems), 256, 0, md->stream>>>(
+        integral_fv_kernel<R><<<grid_for(pd.nitems), 256, 0, st>>>(
             p, m, R(d->cfg.theta), d->cfg.flux_variant, (const R *)d->planes[A][0], (const R *)d->planes[A][1], (const R *)d->planes[A][2],
             (const R *)d->planes[B][0], (const R *)d->planes[B][1], (const R *)d->planes[B][2], pd.d_box, pd.nbox,
             pd.nitems, md->d_int, dts, euler ? 1 : 2);
@@ -872,6 +888,7 @@ int swals_gpu_md_create(swals_domain *const *domains, int32_t ndomains, const do
     }
     auto cleanup = [&](int rc) {
         if (md->pool) cudaFree(md->pool);
+        md->drop_branches();
         delete md;
         return rc;
     };
@@ -1043,7 +1060,14 @@ int swals_gpu_md_create(swals_domain *const *domains, int32_t ndomains, const do
                 return cleanup(api_cuda_fail(ce, "upload"));
         }
     }
-    // All domains run on one stream while they belong to the multidomain.
+    for (int q = 0; ndomains > 1 && q < std::min((int)ndomains, (int)swals_multidomain::BRANCHES); q++) {
+        ce = cudaStreamCreateWithFlags(&md->branch[q], cudaStreamNonBlocking);
+        if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&md->joined[q], cudaEventDisableTiming);
+        if (ce == cudaSuccess && !md->fork) ce = cudaEventCreateWithFlags(&md->fork, cudaEventDisableTiming);
+        if (ce != cudaSuccess) return cleanup(api_cuda_fail(ce, "branch stream"));
+    }
+    // All domains share one stream while they belong to the multidomain (and
+    // leave it only inside a step).
     for (int k = 0; k < ndomains; k++) {
         md->own_streams.push_back(domains[k]->stream);
         domains[k]->stream = md->stream;
@@ -1066,6 +1090,7 @@ int swals_gpu_md_destroy(swals_multidomain *md)
     if (md->graph) cudaGraphDestroy(md->graph);
     for (size_t k = 0; k < md->doms.size(); k++) md->doms[k]->stream = md->own_streams[k];
     if (md->pool) cudaFree(md->pool);
+    md->drop_branches();
     delete md;
     return SWALS_OK;
 }
@@ -1128,29 +1153,52 @@ int swals_gpu_md_evolve_one_step(swals_multidomain *md, double dt)
     const double tend = md->time + dt;
     md_time_begin_kernel<<<1, 1, 0, md->stream>>>(md->d_time, dt);
     md->launches++;
-    for (size_t k = 0; k < md->doms.size(); k++) {
+    const int nd = (int)md->doms.size(), nb = std::min(nd, (int)swals_multidomain::BRANCHES);
+    // Side by side unless a domain's kernels are being timed.
+    bool beside = nd > 1;
+    for (const swals_domain *d : md->doms) beside = beside && !d->timers_on;
+    if (beside) {
+        MDCK(cudaEventRecord(md->fork, md->stream));
+        for (int q = 0; q < nb; q++) MDCK(cudaStreamWaitEvent(md->branch[q], md->fork, 0));
+    }
+    auto advance = [&](int k, cudaStream_t st) -> int {
         swals_domain *d = md->doms[k];
-        int rc = integrals_scale(md, (int)k, 0.0);
+        int rc = integrals_scale(md, k, 0.0, st);
         if (rc) return rc;
         const int nt = md->nt[k];
         const double dt_local = dt / (1.0 * nt);
         for (int s = 0; s < nt; s++) {
-            rc = d->fp64 ? integral_step<double>(md, (int)k, 0, d->cur, dt_local)
-                         : integral_step<float>(md, (int)k, 0, d->cur, dt_local);
+            rc = d->fp64 ? integral_step<double>(md, k, 0, d->cur, dt_local, st)
+                         : integral_step<float>(md, k, 0, d->cur, dt_local, st);
             if (rc) return rc;
             const int A = d->cur;
             rc = swals_gpu_evolve_one_step(d, dt_local, 1);
             if (rc) return rc;
-            rc = d->fp64 ? integral_step<double>(md, (int)k, 1, A, dt_local)
-                         : integral_step<float>(md, (int)k, 1, A, dt_local);
+            rc = d->fp64 ? integral_step<double>(md, k, 1, A, dt_local, st)
+                         : integral_step<float>(md, k, 1, A, dt_local, st);
             if (rc) return rc;
         }
         // domains(j)%time = tend (multidomain_mod.f90:1152)
-        md_time_set_kernel<<<1, 1, 0, md->stream>>>(d->sc, md->d_time);
+        md_time_set_kernel<<<1, 1, 0, st>>>(d->sc, md->d_time);
         md->launches++;
         MDCK(cudaGetLastError());
+        return SWALS_OK;
+    };
+    int rc = SWALS_OK;
+    for (int k = 0; k < nd && rc == SWALS_OK; k++) {
+        cudaStream_t st = beside ? md->branch[k % nb] : md->stream;
+        md->doms[k]->stream = st;   // (md->stream again once it is issued)
+        rc = advance(k, st);
+        md->doms[k]->stream = md->stream;
     }
-    int rc = swals_gpu_md_send_halos(md);
+    if (beside)
+        for (int q = 0; q < nb; q++) {
+            cudaError_t e = cudaEventRecord(md->joined[q], md->branch[q]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(md->stream, md->joined[q], 0);
+            if (e != cudaSuccess && rc == SWALS_OK) rc = api_cuda_fail(e, "joining the domains' branches");
+        }
+    if (rc) return rc;
+    rc = swals_gpu_md_send_halos(md);
     if (rc) return rc;
     rc = swals_gpu_md_recv_halos(md);
     if (rc) return rc;
