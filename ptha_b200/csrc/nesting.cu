@@ -620,8 +620,9 @@ struct swals_multidomain {
     // The domains' sub-steps between two exchanges run side by side, domain k
     // on branch k % BRANCHES, forked from and joined to `stream` every step:
     // they share nothing in between, and their small kernels and last waves
-    // leave most of the chip idle (4 domains of 0.5 - 1.1 million cells, nine
-    // and ten sub-steps: 10.9 -> 8.9 ms for three steps).
+    // leave much of the chip idle (5400 x 1800 leapfrog with nested rk2 grids of
+    // 900^2, 1197 x 801 and 702 x 1098 at 3, 9 and 8 sub-steps: 10.9 -> 8.9 ms
+    // for three steps).
     static constexpr int BRANCHES = 8;
     cudaStream_t branch[BRANCHES] = {};
     cudaEvent_t fork = nullptr, joined[BRANCHES] = {};
