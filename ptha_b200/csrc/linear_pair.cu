@@ -23,7 +23,7 @@
 // row serve the next row too, g dt/area x face depth and the Coriolis factor
 // of a wet face (truly linear solver) both steps, the row constants (dt / area
 // and so on) the whole strip; a segment away from the sides selects nothing.
-// 112 -> about 80 thread instructions a cell and step, 3600 x 2400 FP32
+// 112 -> 93 thread instructions a cell and step, 3600 x 2400 FP32
 // Coriolis 43.7 -> 36.8 us a step.  Products and sums keep the single step's
 // operands and order, so the results are the same bits.
 //
