@@ -73,7 +73,8 @@ __device__ __forceinline__ bool bits_zero(float v) { return __float_as_int(v) ==
 // MC limiter, extrapolation_limiting_mod.f90:63-79 (sign(1,a) == copysign),
 // as the reference writes it, returning TWICE the limited gradient; the edges
 // take U -+ a quarter of it in one fused operation (a product by a power of
-// two is exact, so it rounds as the reference's U -+ 1/2 gradient does).
+// two is exact, but in subnormals, so it rounds as the reference's U -+ 1/2
+// gradient does).
 template <typename R>
 __device__ __forceinline__ R mc_double_gradient_ref(R local, R lower, R upper, R th)
 {
