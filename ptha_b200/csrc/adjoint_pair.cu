@@ -101,21 +101,20 @@ __global__ void __launch_bounds__(32, RESIDENT) adjoint_pair_kernel(const Adjoin
         is_m |= (unsigned)(col >= a.xl + 1 && col <= a.xu - 1) << c;
     }
     // Gauges whose residual this warp's rows and columns receive.
-    const unsigned long long gm =
-        a.ng > 64 ? ~0ull
-                  : pair::sites_in(a.sites, a.ng, strip * OUTC - CPL, strip * OUTC + OUTC + CPL - 1, ra - 2, rb + 1, lane);
+    __shared__ int near[pair::NEAR];
+    const int nnear =
+        pair::sites_near(a.sites, a.ng, strip * OUTC - CPL, strip * OUTC + OUTC + CPL - 1, ra - 2, rb + 1, lane, near);
     auto inject = [&](int row, const double *resid, R(&s)[CPL]) {
-        if (!gm) return;
         auto add = [&](int q) {
             if (a.sites[2 * q + 1] != row) return;
 #pragma unroll
             for (int c = 0; c < CPL; c++)
                 if (a.sites[2 * q] == c0 + c) s[c] = s[c] + R(resid[q]);
         };
-        if (a.ng > 64) {
+        if (nnear > pair::NEAR) {
             for (int q = 0; q < a.ng; q++) add(q);
         } else {
-            for (unsigned long long m = gm; m; m &= m - 1) add(__ffsll((long long)m) - 1);
+            for (int k = 0; k < nnear; k++) add(near[k]);
         }
     };
 

@@ -19,22 +19,27 @@ __device__ __forceinline__ void cp16(void *smem, const void *gmem, int src_bytes
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(src_bytes));
 }
 
-// Of the first 64 sites, those with columns c0 .. c1 and rows r0 .. r1, found
-// by the warp together: two loads a lane instead of a loop over the sites.
-__device__ __forceinline__ unsigned long long sites_in(const int *sites, int n, int c0, int c1, int r0, int r1, int lane)
+// The sites with columns c0 .. c1 and rows r0 .. r1, found by the warp together
+// and listed in their order; each warp looks at all sites once instead of every
+// row's.  More than NEAR of them: `count` says so, and the caller looks at all.
+constexpr int NEAR = 64;
+__device__ __forceinline__ int sites_near(const int *sites, int n, int c0, int c1, int r0, int r1, int lane, int *list)
 {
-    unsigned long long m = 0ull;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int q = lane + 32 * h;
+    int count = 0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+        const int q = q0 + lane;
         bool in = false;
         if (q < n) {
             const int c = sites[2 * q], r = sites[2 * q + 1];
             in = c >= c0 && c <= c1 && r >= r0 && r <= r1;
         }
-        m |= (unsigned long long)__ballot_sync(FULL, in) << (32 * h);
+        const unsigned m = __ballot_sync(FULL, in);
+        const int at = count + __popc(m & ((1u << lane) - 1u));
+        if (in && at < NEAR) list[at] = q;
+        count += __popc(m);
     }
-    return m;
+    __syncwarp();
+    return count;
 }
 
 // Rows per segment (linear_pair.cu): `strips` warps side by side, `resident`
