@@ -476,6 +476,12 @@ int swals_gpu_gauges_read_real4(swals_domain *d, float *out, int32_t max_records
  * the cells the priority mask keeps (all cells without a mask). */
 int swals_gpu_volume_in_priority_domain(swals_domain *d, double *out);
 
+/* The library's straight-line FP64 reciprocal 1/a, quotient a/b and square
+ * root of a on host arrays of n values: correctly rounded for operands and
+ * results between 1e-290 and 1e290 (roots of less, zero included, are zero). */
+enum { SWALS_ROUNDED_RECIPROCAL = 0, SWALS_ROUNDED_QUOTIENT = 1, SWALS_ROUNDED_ROOT = 2 };
+int swals_gpu_rounded(int32_t op, const double *a, const double *b, int64_t n, double *out);
+
 /* Last error message of this thread (util/stop_mod.f90 prints before stopping). */
 int swals_gpu_last_error(char *buf, size_t len);
 /* Library version string. */

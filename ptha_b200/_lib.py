@@ -51,7 +51,7 @@ EXPORTED = [
     "swals_gpu_set_max_U_variables", "swals_gpu_download_max_U",
     "swals_md_build_metadata", "swals_md_metadata_exchanges", "swals_md_metadata_priority",
     "swals_md_metadata_recv_boxes", "swals_md_metadata_free",
-    "swals_gpu_stage_grids_real4", "swals_gpu_gauges_read_real4",
+    "swals_gpu_stage_grids_real4", "swals_gpu_gauges_read_real4", "swals_gpu_rounded",
 ]
 TIMER_NAMES = ["cfl", "fv_stage1", "boundary1", "fv_stage2", "boundary2", "finalize", "leapfrog_edge",
                "leapfrog_step", "gauges", "max_stage"]
@@ -150,6 +150,7 @@ def lib():
         "swals_gpu_batch_tune": [vp, ctypes.POINTER(i32), ctypes.POINTER(dbl)],
         "swals_gpu_batch_set_tile_config": [vp, i32],
         "swals_gpu_batch_tile_config_count": [ctypes.POINTER(i32)],
+        "swals_gpu_rounded": [i32, vp, vp, i64, vp],
         "swals_gpu_adjoint_linear": [vp, i32, dbl, vp, vp, vp],
         "swals_gpu_misfit_gradient_linear": [vp, i32, dbl, vp, i32, ctypes.POINTER(dbl), vp],
         "swals_gpu_volume_interior_noalloc": [vp, vp, vp, i32, i32, i64, i32, i32, vp, vp],

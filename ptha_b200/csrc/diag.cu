@@ -1,6 +1,7 @@
 // diag.cu -- diagnostics reductions: volume_interior and the stationary
-// timestep limits (domain_mod.f90:1815-1849, 1906-1960).
-#include "swals_kernels.h"
+// timestep limits (domain_mod.f90:1815-1849, 1906-1960); the straight-line
+// reciprocal, quotient and root on host arrays.
+#include "domain_internal.h"
 
 #include <cfloat>
 
@@ -9,6 +10,14 @@ namespace {
 
 // One warp per row: fixed-order warp tree of (double)STG - (double)ELV, then
 // one thread adds area(j) * row sum in row order (deterministic).
+__global__ void rounded_kernel(int op, const double *a, const double *b, int64_t n, double *out)
+{
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    out[k] = op == SWALS_ROUNDED_RECIPROCAL ? rcp_ord(a[k]) : op == SWALS_ROUNDED_QUOTIENT ? div_ord(a[k], b[k])
+                                                                                           : sqrt_ord(a[k]);
+}
+
 template <typename R>
 __global__ void row_volume_kernel(int nx, int ny, int64_t P, const R *stg, const R *elv, int n_ext, double *row_sums,
                                   const uint8_t *mask)
@@ -230,3 +239,23 @@ template cudaError_t launch_timestep_max<float>(int, int, int64_t, const float *
                                                 cudaStream_t);
 
 }  // namespace swals
+
+extern "C" int swals_gpu_rounded(int32_t op, const double *a, const double *b, int64_t n, double *out)
+{
+    if (op < SWALS_ROUNDED_RECIPROCAL || op > SWALS_ROUNDED_ROOT || !a || !out || n < 1 || n > (int64_t(1) << 30) ||
+        (op == SWALS_ROUNDED_QUOTIENT && !b))
+        return swals::api_fail(SWALS_ERR_INVALID_ARGUMENT, "bad argument");
+    if (op != SWALS_ROUNDED_QUOTIENT) b = nullptr;
+    const size_t bytes = (size_t)n * sizeof(double);
+    double *d = nullptr;   // a, then b or nothing; the results take the place of a
+    cudaError_t e = cudaMalloc(&d, b ? 2 * bytes : bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && b) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        swals::rounded_kernel<<<(unsigned)((n + 255) / 256), 256>>>(op, d, d + n, n, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? SWALS_OK : swals::api_cuda_fail(e, "swals_gpu_rounded");
+}

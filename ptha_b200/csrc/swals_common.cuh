@@ -35,28 +35,35 @@ template <typename R> __device__ __forceinline__ R rmin(R a, R b) { return (b < 
 template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return (b > a) ? b : a; }
 
 // Correctly rounded FP64 reciprocal, quotient and square root for operands of
-// ordinary size, without a branch: Newton's iteration from the hardware's
-// approximations (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64), then
-// Markstein's final correction from the exact remainder (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34, 1990).  The compiler's own sequences test
-// their operands' range and branch to a general routine; between those
-// branches the scheduler cannot interleave the independent square roots and
-// quotients of an edge, and the stage kernels are bound by exactly that
-// latency.  Here the callers see to the range and use the plain operators
-// outside it: operands, results and remainders between 1e-290 and 1e290, so
-// that nothing overflows, underflows or is infinite.  sqrt_ord takes what is
-// below 1e-290, zero included, as zero.  Compared with the correctly rounded
-// instructions on 2.5e10 operands of each, a quarter of them with
-// significands near 1 or 2: no difference.
-// 1/b within about an ulp.
-__device__ __forceinline__ double rcp_near(double b)
+// ordinary size, without a branch, so that the independent roots and quotients
+// of an edge overlap: the stage kernels are bound by that latency.  From PTX
+// rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 (about 20 bits):
+//   reciprocal: Newton's iteration y <- y + y (1 - b y), every time from the
+//     exact remainder;
+//   quotient: a y corrected twice from its remainder a - b q;
+//   root: Goldschmidt's iteration on g -> sqrt(x) and h -> 1/(2 sqrt(x)),
+//     r = 1/2 - g h, g <- g + g r, h <- h + h r, then the correction
+//     g + h (x - g g).
+// Iterations and last corrections as in P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34 (1990), and "Software division and square root using Goldschmidt's
+// algorithms", Proc. RNC6 (2004).  What a last correction rounds is within
+// 2^-50 ulp of the exact value (2^-53 for reciprocals and quotients), so only
+// results that lie as near to the middle of two neighbours are in doubt; those
+// can be listed from small solutions of A 2^s = B M + c and X 2^s = M^2 - c,
+// and the test of swals_gpu_rounded takes them, the ends of the range and
+// random operands against the correctly rounded operators.
+// The callers see to the range and use the plain operators outside it:
+// operands, results and remainders between 1e-290 and 1e290, so that nothing
+// overflows, underflows or is infinite.  sqrt_ord takes what is below 1e-290,
+// zero included, as zero.
+// A step of Newton's iteration for 1/b.
+__device__ __forceinline__ double rcp_step(double b, double y) { return fma(y, fma(-b, y, 1.0), y); }
+__device__ __forceinline__ double rcp_seed(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = fma(-b, y, 1.0);
-    e = fma(e, e, e);
-    return fma(y, e, y);
+    return y;
 }
 // Markstein's one exception, a significand of b of all ones: 1/b lies just
 // above the middle of 2^k and its successor, and rounds to the latter.
@@ -68,26 +75,30 @@ __device__ __forceinline__ double rcp_of_ones(double b, double y)
 }
 __device__ __forceinline__ double rcp_ord(double b)
 {
-    const double y = rcp_near(b);
-    return rcp_of_ones(b, fma(y, fma(-b, y, 1.0), y));
+    return rcp_of_ones(b, rcp_step(b, rcp_step(b, rcp_step(b, rcp_seed(b)))));
 }
 __device__ __forceinline__ float rcp_ord(float b) { return 1.0f / b; }
 __device__ __forceinline__ double div_ord(double a, double b)
 {
-    const double y = rcp_of_ones(b, rcp_near(b));
-    double q = a * y;
-    q = fma(fma(-b, q, a), y, q);          // within half an ulp and a little
-    return fma(fma(-b, q, a), y, q);       // from its exact remainder
+    const double y1 = rcp_step(b, rcp_seed(b));
+    const double y = rcp_of_ones(b, rcp_step(b, y1));
+    double q = a * y1;
+    q = fma(fma(-b, q, a), y1, q);
+    return fma(fma(-b, q, a), y, q);
 }
 __device__ __forceinline__ double sqrt_ord(double x)
 {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    y = fma(fma(0.375, e, 0.5), y * e, y);
-    const double g = x * y;
-    const double r = fma(fma(-g, g, x), 0.5 * y, g);
-    return (x < 1.0e-290) ? 0.0 : r;
+    double g = x * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    g = fma(fma(-g, g, x), h, g);
+    return (x < 1.0e-290) ? 0.0 : g;
 }
 __device__ __forceinline__ float sqrt_ord(float x) { return sqrtf(x); }
 
