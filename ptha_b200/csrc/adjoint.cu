@@ -436,11 +436,20 @@ int adjoint_steps(swals_domain *d, R *const lam[2][3], int c, int count, double 
     return c;
 }
 
-// The domain's adjoint scratch, grown to at least `need` bytes.
+void drop_adjoint_graphs(swals_domain *d)
+{
+    for (auto &g : d->adj_graph)
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    d->adj_K = 0;
+}
+
+// The domain's adjoint scratch, grown to at least `need` bytes; the graphs of
+// misfit_gradient hold addresses in it and go with it.
 cudaError_t workspace(swals_domain *d, size_t need, void **out)
 {
     if (d->ws_bytes < need) {
         cudaStreamSynchronize(d->stream);
+        drop_adjoint_graphs(d);
         if (d->ws) cudaFree(d->ws);
         d->ws = nullptr;
         d->ws_bytes = 0;
@@ -632,6 +641,8 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     const int64_t plane = d->pitch * (int64_t)d->ny;
     const size_t es = sizeof(R);
     const int nseg = (nsteps + K - 1) / K;
+    // What the replayed graphs address (planes, records, residuals, sites) comes
+    // first and lies alike for every nsteps; what depends on nsteps follows.
     size_t need = (size_t)(6 + 12 + 3 * nseg) * plane * es;          // lambda x2, state x2 x2 sets, checkpoints
     need += sizeof(double) * ((size_t)nsteps * ng + 4 * (size_t)K * ng + (size_t)nsteps + 8);
     need += sizeof(int) * 2 * (size_t)ng + 1024;
@@ -645,14 +656,15 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     for (int q = 0; q < 2; q++)
         for (int b = 0; b < 2; b++)
             for (int v = 0; v < 3; v++) { xs[q][b][v] = (R *)p; p += plane * es; }
-    R *ckpt = (R *)p; p += (size_t)3 * nseg * plane * es;
-    double *d_target = (double *)p; p += sizeof(double) * (size_t)nsteps * ng;
     double *d_rec[2], *d_resid[2];
     for (int q = 0; q < 2; q++) { d_rec[q] = (double *)p; p += sizeof(double) * (size_t)K * ng; }
     for (int q = 0; q < 2; q++) { d_resid[q] = (double *)p; p += sizeof(double) * (size_t)K * ng; }
+    int *d_sites = (int *)p; p += sizeof(int) * 2 * (size_t)ng;
+    double *d_target = (double *)p; p += sizeof(double) * (size_t)nsteps * ng;
     double *d_half = (double *)p; p += sizeof(double) * (size_t)nsteps;
     double *d_loss = (double *)p; p += sizeof(double) * 8;
-    int *d_sites = (int *)p;
+    p += (256 - (uintptr_t)p % 256) % 256;
+    R *ckpt = (R *)p;
 
     int rc = SWALS_OK;
     auto ck = [&](cudaError_t err, const char *w) { if (err != cudaSuccess && rc == SWALS_OK) rc = swals::api_cuda_fail(err, w); };
@@ -692,9 +704,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     };
     const bool graphs = (K % 2 == 0) && K <= nsteps && !d->timers_on;
     if (graphs && (d->adj_K != K || d->adj_ng != ng || d->adj_dt != dt || d->adj_ws != d->ws || !d->adj_graph[0])) {
-        for (auto &g : d->adj_graph)
-            if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-        d->adj_K = 0;
+        drop_adjoint_graphs(d);
         const int64_t l0 = d->launches;
         for (int q = 0; q < 7 && rc == SWALS_OK; q++) {
             ck(cudaStreamBeginCapture(d->stream, cudaStreamCaptureModeThreadLocal), "capture");
