@@ -713,14 +713,20 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
             else adj_seq(K, (q - 2) % 3, (q - 2) / 3);
             cudaGraph_t gr = nullptr;
             ck(cudaStreamEndCapture(d->stream, &gr), "end capture");
+            d->adj_launches[q] = d->launches - l0;
+            d->launches = l0;
             if (gr) {
                 ck(cudaGraphInstantiate(&d->adj_graph[q], gr, 0), "instantiate");
                 cudaGraphDestroy(gr);
             }
         }
-        d->launches = l0;
         if (rc == SWALS_OK) { d->adj_K = K; d->adj_ng = ng; d->adj_dt = dt; d->adj_ws = d->ws; }
     }
+
+    auto replay = [&](int q, cudaStream_t st, const char *w) {
+        ck(cudaGraphLaunch(d->adj_graph[q], st), w);
+        d->launches += d->adj_launches[q];
+    };
 
     // Forward sweep with checkpoints, up to the last one: nothing reads the
     // states after it but its own recomputation.
@@ -732,8 +738,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
                                cudaMemcpyDeviceToDevice, d->stream), "checkpoint");
         if (sgm == nseg - 1) break;
         if (graphs && cnt == K && cur == 0) {
-            ck(cudaGraphLaunch(d->adj_graph[0], d->stream), "forward graph");
-            d->launches += K;
+            replay(0, d->stream, "forward graph");
         } else {
             cur = fwd_seq(cnt, cur);
         }
@@ -746,8 +751,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
             ck(cudaMemcpyAsync(xs[set][0][v], ckpt + ((size_t)sgm * 3 + v) * plane, plane * es,
                                cudaMemcpyDeviceToDevice, st), "restore");
         if (graphs && cnt == K) {
-            ck(cudaGraphLaunch(d->adj_graph[1 + 3 * set], st), "recompute graph");
-            d->launches += K;
+            replay(1 + 3 * set, st, "recompute graph");
         } else {
             rec_seq(cnt, set, st);
         }
@@ -775,8 +779,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
             if (overlap) ck(cudaEventRecord(d->aux.join, st), "join");
         }
         if (graphs && cnt == K) {
-            ck(cudaGraphLaunch(d->adj_graph[2 + 3 * set + lc], d->stream), "adjoint graph");
-            d->launches += K;
+            replay(2 + 3 * set + lc, d->stream, "adjoint graph");
         } else {
             lc = adj_seq(cnt, lc, set);
         }

@@ -83,6 +83,7 @@ struct swals_domain {
     // [0] forward; [1 + 3 set] recompute into buffer set `set`;
     // [2 + 3 set + lc] adjoint from lambda buffer lc with set's residuals
     cudaGraphExec_t adj_graph[7] = {};
+    int64_t adj_launches[7] = {};   // kernels in each
     int adj_K = 0, adj_ng = 0;
     double adj_dt = 0.0;
     void *adj_ws = nullptr;

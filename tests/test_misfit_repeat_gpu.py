@@ -44,3 +44,23 @@ def test_each_call_equals_a_fresh_domain(real_bytes):
             assert loss == loss1 and loss > 0.0, (k, nsteps)
             np.testing.assert_array_equal(g, g1, err_msg=str((k, nsteps)))
             assert np.isfinite(g).all() and np.abs(g).max() > 0.0
+
+
+@pytest.mark.parametrize("every", [20, 22, 10])
+def test_launches_counted_as_launched(every):
+    """A replayed segment counts the kernels it holds: as many as when every
+    kernel is launched by itself (timers on)."""
+    kw, U = workloads.spherical_patch(nx=NX, ny=NY, seed=3)
+    kw.update(timestepping_method="linear")
+    target = np.zeros((100, NG))
+    with Domain(**kw) as d:
+        d.set_U(U)
+        d.gauges_setup(_sites(kw, 0), 200)
+        dt = 0.8 * d.linear_timestep_max()
+        counts = []
+        for timed in (False, False, True):
+            d.timers_enable(timed)
+            n = d.launch_count()
+            d.misfit_gradient(100, dt, target, checkpoint_every=every)
+            counts.append(d.launch_count() - n)
+    assert counts[0] == counts[1] == counts[2] > 0
