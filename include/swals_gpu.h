@@ -236,12 +236,16 @@ int swals_gpu_batch_gauges_setup(swals_batch *b, const double *xy, int32_t n, in
 int swals_gpu_batch_gauges_read(swals_batch *b, double *out, int32_t max_records, int32_t *n_records);
 int swals_gpu_batch_evolve(swals_batch *b, int32_t nsteps, double dt);
 int swals_gpu_batch_time(swals_batch *b, double *time, int64_t *nsteps);
-/* Autotuner: times every tile shape on this batch with state-preserving
- * dt = 0 steps and keeps the fastest. */
+/* Autotuner: times every kernel of a single step and the pass that takes two
+ * steps on this batch, with state-preserving dt = 0 steps, and keeps the
+ * fastest, in place of an earlier choice.  cfg_out is the fastest kernel of a
+ * single step (where the two-step pass wins, an odd last step takes it),
+ * ms_per_step_out the time a step of what evolve then uses. */
 int swals_gpu_batch_tune(swals_batch *b, int32_t *cfg_out, double *ms_per_step_out);
+/* Every step by kernel cfg, one at a time. */
 int swals_gpu_batch_set_tile_config(swals_batch *b, int32_t cfg);
-/* Number of kernel configurations the autotuner chooses from (valid cfg
- * values of swals_gpu_batch_set_tile_config are 0 .. n-1). */
+/* Number of kernels of a single step (valid cfg values of
+ * swals_gpu_batch_set_tile_config are 0 .. n-1). */
 int swals_gpu_batch_tile_config_count(int32_t *n);
 
 /* ---- discrete adjoint of the truly linear leapfrog -------------------------

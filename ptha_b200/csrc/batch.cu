@@ -27,7 +27,7 @@ struct swals_batch {
     double time = 0.0;
     int64_t nsteps = 0;
     int tile_cfg = 0;         // kernel of a single step
-    bool tile_set = false;    // chosen by the caller: every step takes it, one at a time
+    bool tile_set = false;    // every step takes it, one at a time: chosen by the caller or the tuner
     // gauges
     int n_gauges = 0, capacity = 0, nrec = 0;
     int *d_sites = nullptr;
@@ -164,13 +164,11 @@ bool pair_fits(const swals_batch *b)
     return swals::linear_pair_fits<R>(p, b->inst_stride, b->plane);
 }
 
-// Two steps at a time unless the caller chose a kernel: 12 instances of 1800 x
+// Two steps at a time unless a kernel of single steps was chosen: 12 instances of 1800 x
 // 1200 FP32 with Coriolis and 50 gauges, 120 steps and the copy of max_stage:
 // 26.5 ms by the best single-step kernel, 15.5 in pairs.
-bool takes_pairs(const swals_batch *b)
-{
-    return !b->tile_set && (b->grid->fp64 ? pair_fits<double>(b) : pair_fits<float>(b));
-}
+bool can_pair(const swals_batch *b) { return b->grid->fp64 ? pair_fits<double>(b) : pair_fits<float>(b); }
+bool takes_pairs(const swals_batch *b) { return !b->tile_set && can_pair(b); }
 
 void drop_graph(swals_batch *b)
 {
@@ -445,30 +443,43 @@ int swals_gpu_batch_tune(swals_batch *b, int32_t *cfg_out, double *ms_per_step_o
     cudaEvent_t e0, e1;
     BCK(cudaEventCreate(&e0));
     BCK(cudaEventCreate(&e1));
-    const int ncfg = swals::linear_tile_config_count();
-    int best = 0;
-    float best_ms = 1e30f;
-    const int saved = b->tile_cfg;
-    for (int c = 0; c < ncfg; c++) {
-        b->tile_cfg = c;
-        // dt = 0 steps leave the state unchanged but move the same bytes and
-        // do the same arithmetic; an even count keeps the buffer parity.
-        for (int k = 0; k < 2; k++) BCK(step_any(b, 0.0, false));
+    // Six launches of a form after two of warming up, in ms.  dt = 0 steps
+    // leave the state unchanged but move the same bytes and do the same
+    // arithmetic; an even count keeps the buffer parity.
+    auto time_six = [&](cudaError_t (*form)(swals_batch *, double, bool), float &ms) -> int {
+        for (int k = 0; k < 2; k++) BCK(form(b, 0.0, false));
         BCK(cudaEventRecord(e0, g->stream));
-        for (int k = 0; k < 6; k++) BCK(step_any(b, 0.0, false));
+        for (int k = 0; k < 6; k++) BCK(form(b, 0.0, false));
         BCK(cudaEventRecord(e1, g->stream));
         BCK(cudaEventSynchronize(e1));
-        float ms = 0.f;
         BCK(cudaEventElapsedTime(&ms, e0, e1));
+        return SWALS_OK;
+    };
+    const int ncfg = swals::linear_tile_config_count();
+    int best = 0, rc = SWALS_OK;
+    float best_ms = 1e30f;
+    for (int c = 0; c < ncfg && rc == SWALS_OK; c++) {
+        b->tile_cfg = c;
+        float ms = 0.f;
+        rc = time_six(step_any, ms);
         if (ms < best_ms) { best_ms = ms; best = c; }
     }
-    (void)saved;
+    double ms_per_step = best_ms / 6.0;
     b->tile_cfg = best;
-    b->tile_set = false;   // (it is for the steps that do not pair)
+    b->tile_set = true;
+    if (rc == SWALS_OK && can_pair(b)) {   // two steps a launch
+        float ms = 0.f;
+        rc = time_six(two_any, ms);
+        if (ms / 12.0 < ms_per_step) {
+            ms_per_step = ms / 12.0;
+            b->tile_set = false;
+        }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (rc) return rc;
     if (cfg_out) *cfg_out = best;
-    if (ms_per_step_out) *ms_per_step_out = best_ms / 6.0;
+    if (ms_per_step_out) *ms_per_step_out = ms_per_step;
     return SWALS_OK;
 }
 
