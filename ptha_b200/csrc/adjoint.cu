@@ -503,7 +503,8 @@ int adjoint_sweep(swals_domain *d, int nsteps, double dt, const double *gadj_hos
     const size_t es = sizeof(R);
     const int ng = d->n_gauges > 0 ? d->n_gauges : (int)(d->h_sites.size() / 2);
     void *buf = nullptr;
-    const size_t need = 6 * plane * es + sizeof(double) * (size_t)nsteps * (ng > 0 ? ng : 1) + 2 * sizeof(int) * (ng + 1);
+    const size_t need = 6 * plane * es + sizeof(double) * (size_t)nsteps * (ng > 0 ? ng : 1) +
+                        sizeof(int) * d->h_index.size();
     cudaError_t e = workspace(d, need, &buf);
     if (e != cudaSuccess) return swals::api_cuda_fail(e, "adjoint workspace");
     R *lam[2][3];
@@ -516,7 +517,8 @@ int adjoint_sweep(swals_domain *d, int nsteps, double dt, const double *gadj_hos
     if (e == cudaSuccess && ng > 0) {
         e = cudaMemcpyAsync(d_g, gadj_host, sizeof(double) * (size_t)nsteps * ng, cudaMemcpyHostToDevice, d->stream);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_sites, d->h_sites.data(), sizeof(int) * 2 * ng, cudaMemcpyHostToDevice, d->stream);
+            e = cudaMemcpyAsync(d_sites, d->h_index.data(), sizeof(int) * d->h_index.size(), cudaMemcpyHostToDevice,
+                                d->stream);
     }
     if (e != cudaSuccess) rc = swals::api_cuda_fail(e, "adjoint setup");
     int cur = 0;
@@ -645,7 +647,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     // first and lies alike for every nsteps; what depends on nsteps follows.
     size_t need = (size_t)(6 + 12 + 3 * nseg) * plane * es;          // lambda x2, state x2 x2 sets, checkpoints
     need += sizeof(double) * ((size_t)nsteps * ng + 4 * (size_t)K * ng + (size_t)nsteps + 8);
-    need += sizeof(int) * 2 * (size_t)ng + 1024;
+    need += sizeof(int) * d->h_index.size() + 1024;
     void *buf = nullptr;
     cudaError_t e = workspace(d, need, &buf);
     if (e != cudaSuccess) return swals::api_cuda_fail(e, "misfit-gradient workspace");
@@ -659,7 +661,7 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     double *d_rec[2], *d_resid[2];
     for (int q = 0; q < 2; q++) { d_rec[q] = (double *)p; p += sizeof(double) * (size_t)K * ng; }
     for (int q = 0; q < 2; q++) { d_resid[q] = (double *)p; p += sizeof(double) * (size_t)K * ng; }
-    int *d_sites = (int *)p; p += sizeof(int) * 2 * (size_t)ng;
+    int *d_sites = (int *)p; p += sizeof(int) * d->h_index.size();
     double *d_target = (double *)p; p += sizeof(double) * (size_t)nsteps * ng;
     double *d_half = (double *)p; p += sizeof(double) * (size_t)nsteps;
     double *d_loss = (double *)p; p += sizeof(double) * 8;
@@ -678,7 +680,8 @@ int misfit_gradient(swals_domain *d, int nsteps, double dt, const double *target
     ck(cudaMemsetAsync(lam[0][0], 0, 3 * plane * es, d->stream), "memset");
     ck(cudaMemcpyAsync(d_target, target_host, sizeof(double) * (size_t)nsteps * ng, cudaMemcpyHostToDevice, d->stream),
        "target upload");
-    ck(cudaMemcpyAsync(d_sites, d->h_sites.data(), sizeof(int) * 2 * ng, cudaMemcpyHostToDevice, d->stream), "sites");
+    ck(cudaMemcpyAsync(d_sites, d->h_index.data(), sizeof(int) * d->h_index.size(), cudaMemcpyHostToDevice, d->stream),
+       "sites");
     for (int v = 0; v < 3; v++)
         ck(cudaMemcpyAsync(xs[0][0][v], d->planes[d->cur][v], plane * es, cudaMemcpyDeviceToDevice, d->stream), "x0");
 

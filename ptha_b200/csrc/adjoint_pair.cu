@@ -80,8 +80,9 @@ __global__ void __launch_bounds__(32, RESIDENT) adjoint_pair_kernel(const Adjoin
         c.w1 = c.cr * a.m.dxb[r + 1];
         rc[k] = c;
     }
+    const pair::GaugeRows gauges(reinterpret_cast<int *>(rc + (SH + 4)), a.sites, a.ng, ny, ra - 2, rb - ra + 4, lane);
     __syncwarp();
-    after_previous();   // (the metrics above are no kernel's output)
+    after_previous();   // (the metrics and gauge sites above are no kernel's output)
     let_next_start();
 
     const int c0 = strip * OUTC + (lane - 1) * CPL;          // this lane's first column
@@ -100,22 +101,22 @@ __global__ void __launch_bounds__(32, RESIDENT) adjoint_pair_kernel(const Adjoin
         im_m |= (unsigned)(col >= a.xl && col <= a.xu - 1) << c;
         is_m |= (unsigned)(col >= a.xl + 1 && col <= a.xu - 1) << c;
     }
-    // Gauges whose residual this warp's rows and columns receive.
-    __shared__ int near[pair::NEAR];
-    const int nnear =
-        pair::sites_near(a.sites, a.ng, strip * OUTC - CPL, strip * OUTC + OUTC + CPL - 1, ra - 2, rb + 1, lane, near);
+    // The gauges in the warp's columns, halo included; a cell may have several,
+    // added in their order.
     auto inject = [&](int row, const double *resid, R(&s)[CPL]) {
-        auto add = [&](int q) {
-            if (a.sites[2 * q + 1] != row) return;
+        if (a.ng <= 0) return;
+        gauges.on_row(row - (ra - 2), strip * OUTC - CPL, strip * OUTC + OUTC + CPL - 1, lane,
+                      [&](unsigned m, bool hit, int col, int q) {
+            const R g = hit ? R(resid[q]) : zero;
+            for (; m; m &= m - 1) {
+                const int k = __ffs(m) - 1;
+                const int at = __shfl_sync(FULL, col, k) - lane * CPL;
+                const R gk = __shfl_sync(FULL, g, k);
 #pragma unroll
-            for (int c = 0; c < CPL; c++)
-                if (a.sites[2 * q] == c0 + c) s[c] = s[c] + R(resid[q]);
-        };
-        if (nnear > pair::NEAR) {
-            for (int q = 0; q < a.ng; q++) add(q);
-        } else {
-            for (int k = 0; k < nnear; k++) add(near[k]);
-        }
+                for (int c = 0; c < CPL; c++)
+                    if (at == c) s[c] = s[c] + gk;
+            }
+        });
     };
 
     const int r0 = max(ra - 2, 0);
@@ -322,7 +323,7 @@ cudaError_t launch_adjoint_pair(const AdjointPair<R> &a, bool coriolis, cudaStre
     const int nstrips = (a.nx + 30 * CPL - 1) / (30 * CPL);
     const int sh = pair::rows(nstrips, a.ny, RESIDENT, false);
     const unsigned ctas = (unsigned)(nstrips * ((a.ny + sh - 1) / sh));
-    const size_t smem = 16 * (32 * NP + 1) * SLOTS + sizeof(RowConst<R>) * (sh + 4);
+    const size_t smem = 16 * (32 * NP + 1) * SLOTS + sizeof(RowConst<R>) * (sh + 4) + (a.ng > 0 ? 4 * (sh + 5) : 0);
     if (coriolis) return launch_behind(adjoint_pair_kernel<R, true>, ctas, 32, smem, s, a, sh, nstrips);
     return launch_behind(adjoint_pair_kernel<R, false>, ctas, 32, smem, s, a, sh, nstrips);
 }

@@ -348,8 +348,9 @@ int swals_gpu_batch_gauges_setup(swals_batch *b, const double *xy, int32_t n, in
         }
     }
     if (n > 0) {
-        BCK(cudaMalloc(&b->d_sites, sizeof(int) * 2 * (size_t)n));
-        BCK(cudaMemcpy(b->d_sites, b->h_sites.data(), sizeof(int) * 2 * (size_t)n, cudaMemcpyHostToDevice));
+        const std::vector<int> index = swals::sites_with_index(b->h_sites, g->ny);
+        BCK(cudaMalloc(&b->d_sites, sizeof(int) * index.size()));
+        BCK(cudaMemcpy(b->d_sites, index.data(), sizeof(int) * index.size(), cudaMemcpyHostToDevice));
         if (capacity > 0) BCK(cudaMalloc(&b->d_records, sizeof(double) * (size_t)n * b->nbatch * capacity));
     }
     b->n_gauges = capacity > 0 ? n : 0;

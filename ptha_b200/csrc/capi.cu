@@ -8,11 +8,13 @@
 // on the device; the host only keeps descriptors and the 1-D metrics.
 #include "domain_internal.h"
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -223,6 +225,27 @@ void on_launch(void *ctx, int cat, int phase)
 }
 
 }  // namespace
+
+std::vector<int> swals::sites_with_index(const std::vector<int> &sites, int ny)
+{
+    const int n = (int)sites.size() / 2;
+    std::vector<int> order(n), out(sites);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return sites[2 * a + 1] != sites[2 * b + 1] ? sites[2 * a + 1] < sites[2 * b + 1] : sites[2 * a] < sites[2 * b];
+    });
+    out.resize(4 * (size_t)n + gauge_index_rows(ny), n);
+    int *row_start = out.data() + 2 * (size_t)n, *sorted = row_start + gauge_index_rows(ny);
+    for (int r = 0, k = 0; r <= ny; r++) {
+        while (k < n && sites[2 * order[k] + 1] < r) k++;
+        row_start[r] = k;
+    }
+    for (int k = 0; k < n; k++) {
+        sorted[2 * k] = sites[2 * order[k]];
+        sorted[2 * k + 1] = order[k];
+    }
+    return out;
+}
 
 swals::LaunchHook swals::hook_of(swals_domain *d)
 {
@@ -1249,7 +1272,9 @@ int swals_gpu_gauges_setup(swals_domain *d, const double *xy, int32_t n, int32_t
     if (d->d_sites) { cudaFree(d->d_sites); d->d_sites = nullptr; }
     if (d->d_records) { cudaFree(d->d_records); d->d_records = nullptr; }
     d->n_gauges = 0;
-    d->h_sites.assign(2 * (size_t)n, 0);
+    d->h_sites.clear();
+    d->h_index.clear();
+    std::vector<int> sites(2 * (size_t)n);
     // point_gauge_mod.f90:336-347, evaluated in the state precision
     const double dx[2] = {d->desc.lw[0] / d->nx, d->desc.lw[1] / d->ny};
     const int nxy[2] = {d->nx, d->ny};
@@ -1267,12 +1292,14 @@ int swals_gpu_gauges_setup(swals_domain *d, const double *xy, int32_t n, int32_t
             if (site < 1 || site > nxy[k])
                 return fail(SWALS_ERR_INVALID_ARGUMENT, "Gauge coordinate (%g, %g) is outside the domain",
                             xy[2 * g], xy[2 * g + 1]);
-            d->h_sites[2 * g + k] = site - 1;
+            sites[2 * g + k] = site - 1;
         }
     }
     if (n > 0) {
-        CK(cudaMalloc(&d->d_sites, sizeof(int) * 2 * (size_t)n));
-        CK(cudaMemcpy(d->d_sites, d->h_sites.data(), sizeof(int) * 2 * (size_t)n, cudaMemcpyHostToDevice));
+        d->h_sites = sites;
+        d->h_index = swals::sites_with_index(sites, d->ny);
+        CK(cudaMalloc(&d->d_sites, sizeof(int) * d->h_index.size()));
+        CK(cudaMemcpy(d->d_sites, d->h_index.data(), sizeof(int) * d->h_index.size(), cudaMemcpyHostToDevice));
         if (capacity > 0) CK(cudaMalloc(&d->d_records, sizeof(double) * 3 * (size_t)n * capacity));
     }
     d->n_gauges = (capacity > 0) ? n : 0;

@@ -47,7 +47,7 @@ struct swals_domain {
     int n_gauges = 0, gauge_capacity = 0;
     int *d_sites = nullptr;
     double *d_records = nullptr;
-    std::vector<int> h_sites;
+    std::vector<int> h_sites, h_index;   // (i, j); the same and their index, as on the device
     // launch accounting and per-kernel event timers
     int64_t launches = 0;
     // Diagnostics: the domain's own priority cells (nx*ny bytes, i fastest)

@@ -110,8 +110,10 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
         c.dtj = COR ? dt * a.m.cor_be[r + 1] * half : zero;
         rc[k] = c;
     }
+    const pair::GaugeRows gauges(reinterpret_cast<int *>(rc + (SH + 4)), a.g_sites, GAUGES ? a.g_n : 0, ny, ra - 2,
+                                 rb - ra + 4, lane);
     __syncthreads();
-    after_previous();   // (the metrics above are no kernel's output)
+    after_previous();   // (the metrics and gauge sites above are no kernel's output)
     let_next_start();
     const int rec = GAUGES ? (a.g_count ? *a.g_count : 0) : 0;
 
@@ -136,27 +138,29 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
         mo_m |= (unsigned)(col >= a.xl && col <= a.xu - 1) << c;
         ms_m |= (unsigned)(col >= a.xl && col <= a.xu) << c;
     }
-    // gauges in the warp's output columns and rows
-    __shared__ int near[GAUGES ? pair::NEAR : 1];
-    const int nnear =
-        GAUGES ? pair::sites_near(a.g_sites, a.g_n, strip * OUTC, strip * OUTC + OUTC - 1, ra, rb - 1, lane, near) : 0;
+    // the gauges in the warp's output columns
     auto record = [&](int step, int row, const R(&s)[CPL], const R(&u)[CPL], const R(&v)[CPL]) {
         if (rec + step >= a.g_capacity) return;
-        auto put = [&](int q) {
+        gauges.on_row(row - (ra - 2), strip * OUTC, strip * OUTC + OUTC - 1, lane, [&](unsigned, bool hit, int col, int q) {
+            // the lane with the site fetches the values of its cell
+            const int from = 1 + col / CPL, comp = col % CPL;
+            auto fetch = [&](const R(&x)[CPL]) {
+                R y = __shfl_sync(FULL, x[0], from);
 #pragma unroll
-            for (int c = 0; c < CPL; c++)
-                if (a.g_sites[2 * q] == c0 + c && a.g_sites[2 * q + 1] == row) {
-                    double *d = a.g_rec + (((int64_t)(rec + step) * a.nbatch + b) * a.g_n + q) * a.g_vals;
-                    d[0] = (double)s[c];
-                    if (a.g_vals == 3) { d[1] = (double)u[c]; d[2] = (double)v[c]; }
+                for (int c = 1; c < CPL; c++) {
+                    const R z = __shfl_sync(FULL, x[c], from);
+                    if (comp == c) y = z;
                 }
-        };
-        if (!out) return;
-        if (nnear > pair::NEAR) {
-            for (int q = 0; q < a.g_n; q++) put(q);
-        } else {
-            for (int k = 0; k < nnear; k++) put(near[k]);
-        }
+                return (double)y;
+            };
+            double *d = a.g_rec + (((int64_t)(rec + step) * a.nbatch + b) * a.g_n + q) * a.g_vals;
+            const double fs = fetch(s);
+            if (hit) d[0] = fs;
+            if (a.g_vals == 3) {
+                const double fu = fetch(u), fv = fetch(v);
+                if (hit) { d[1] = fu; d[2] = fv; }
+            }
+        });
     };
     // the lane's component on the west and east boundary-flux lines, or -1
     const int ln_e = (a.lines && out) ? nx - a.n_ext - 1 - c0 : -1, ln_w = (a.lines && out) ? a.n_ext - 1 - c0 : -1;
@@ -402,8 +406,8 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
                             if (max_stage) max_stage[o + c] = m[c];
                         }
                 }
-                if (GAUGES) record(1, q, b2, uB, vB);
             }
+            if (GAUGES && q >= ra) record(1, q, b2, uB, vB);
 #pragma unroll
             for (int c = 0; c < CPL; c++) {
                 e2[c] = e1[c];
@@ -509,7 +513,8 @@ cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
     const int nstrips = (a.p.nx + 30 * CPL - 1) / (30 * CPL);
     const int sh = pair::rows((int64_t)nstrips * a.nbatch, a.p.ny, pair_warps(NLF, (int)sizeof(R)), NLF);
     const int64_t ctas = (int64_t)nstrips * ((a.p.ny + sh - 1) / sh) * a.nbatch;
-    const size_t smem = 16 * 32 * (NLF ? 7 : 5) * SLOTS + sizeof(RowConst<R>) * (sh + 4);
+    const size_t smem =
+        16 * 32 * (NLF ? 7 : 5) * SLOTS + sizeof(RowConst<R>) * (sh + 4) + (a.g_n > 0 ? 4 * (sh + 5) : 0);
     auto go = [&](auto kernel) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         if (e != cudaSuccess) return e;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "swals_common.cuh"
 
@@ -195,6 +196,12 @@ template <typename R>
 cudaError_t launch_linear_map(const StepPlanes<R> &p, const Metrics<R> &m, const StepConfig &c, R dt,
                               const int *sites, int n_sites, double *rec, cudaStream_t s, const LaunchHook &hook);
 
+// Gauge sites (i, j) on the device are followed by an index of them by row, for
+// the two-steps-a-pass kernels: where each row's sites start, gauge_index_rows
+// ints, then (column, gauge) sorted by row, column, gauge.
+__host__ __device__ inline int gauge_index_rows(int ny) { return (ny + 2) / 2 * 2; }   // ny + 1, 8-byte steps
+std::vector<int> sites_with_index(const std::vector<int> &sites, int ny);
+
 // Two linear leapfrog steps in one pass (linear_pair.cu): p's output planes
 // hold the state two steps on.  Plain steps only (no boundary routine, no
 // forcing), on planes that linear_pair_fits accepts.  The caller fills the
@@ -211,7 +218,7 @@ struct LinearPair {
     int64_t inst_stride, max_stride;   // elements between instances' planes, max_stage planes
     const R *fw;            // friction work (UH points, then fw_plane elements on the VH points) or null
     int64_t fw_plane;
-    // Gauges: sites (i, j), record (count + step) of each instance, g_vals = 3
+    // Gauges: sites (i, j) and their index, record (count + step) of each instance, g_vals = 3
     // (stage, UH, VH) or 1 (stage) values; the last CTA adds two to *g_count.
     // A null g_count stands for 0 and is not advanced.
     const int *g_sites;
@@ -243,7 +250,7 @@ struct AdjointPair {
     Metrics<R> m;
     int xl, xu, yl, yu;
     R dt, msl, mult;         // mult: linear friction factor (1 without friction)
-    const int *sites;        // ng gauge cells (i, j); ng = 0: none
+    const int *sites;        // ng gauge cells (i, j) and their index; ng = 0: none
     int ng;
     const double *resid, *resid2;
 };
