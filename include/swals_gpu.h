@@ -177,7 +177,8 @@ int swals_gpu_gauges_reset(swals_domain *d);
  * ms_out[2c] = total milliseconds and ms_out[2c+1] = number of launches;
  * categories: 0 CFL pre-pass, 1 FV stage 1, 2 boundary after stage 1,
  * 3 FV stage 2 (+rk2 average), 4 boundary after stage 2, 5 step finalise,
- * 6 leapfrog edge/boundary, 7 leapfrog fused step, 8 gauges, 9 max_stage. */
+ * 6 leapfrog edge/boundary, 7 leapfrog fused step (evolve_steps: the pass that
+ * takes two), 8 gauges, 9 max_stage. */
 #define SWALS_TIMER_CATEGORIES 10
 int swals_gpu_timers_enable(swals_domain *d, int32_t enable);
 int swals_gpu_timers_read(swals_domain *d, double *ms_out, int32_t n, int32_t *n_written);

@@ -756,7 +756,8 @@ namespace {
 
 // Two plain linear steps of fixed dt by one pass (linear_pair.cu), `pair`-th
 // of a sequence; their bookkeeping follows on the side stream, beside the
-// next pair.  A line buffer and a state buffer are written again two and three
+// next pair (with timers on, on the domain's stream, where their events are).
+// A line buffer and a state buffer are written again two and three
 // pairs on, after the bookkeeping that reads them (pair_edge).
 template <typename R>
 swals::LinearPair<R> pair_args(swals_domain *d, double timestep, int pair)
@@ -788,8 +789,7 @@ swals::LinearPair<R> pair_args(swals_domain *d, double timestep, int pair)
 bool takes_pairs(const swals_domain *d, int has_dt)
 {
     const bool lf = d->method == M_LINEAR || (d->method == M_LF_LIN_NLFRIC && d->cfg.truely_linear);
-    if (!lf || !has_dt || d->cfg.bc_kind != SWALS_BC_NONE || d->cfg.n_forcing || d->timers_on || d->static_pending)
-        return false;
+    if (!lf || !has_dt || d->cfg.bc_kind != SWALS_BC_NONE || d->cfg.n_forcing || d->static_pending) return false;
     if (d->desc.record_max_stage && (d->max_U_update_frequency > 1 || d->max_u_generic)) return false;
     const char *e = getenv("SWALS_LINEAR_KERNEL");
     if (e && *e && strcmp(e, "pair") != 0) return false;
@@ -804,22 +804,26 @@ int evolve_pairs_t(swals_domain *d, double timestep, int npairs)
     for (cudaEvent_t *e : {&d->pair_main, &d->pair_edge[0], &d->pair_edge[1]})
         if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     const swals::LaunchHook hook = swals::hook_of(d);
+    const bool beside = !d->timers_on;
+    const cudaStream_t es = beside ? d->aux.stream : d->stream;
     for (int k = 0; k < npairs; k++) {
         const swals::LinearPair<R> a = pair_args<R>(d, timestep, k);
-        if (k >= 2) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[k & 1], 0));
+        if (beside && k >= 2) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[k & 1], 0));
         hook(swals::CAT_LINEAR_MAIN, 0);
         CK(swals::launch_linear_pair<R>(a, d->cfg, d->stream));
         hook(swals::CAT_LINEAR_MAIN, 1);
-        CK(cudaEventRecord(d->pair_main, d->stream));
-        CK(cudaStreamWaitEvent(d->aux.stream, d->pair_main, 0));
+        if (beside) {
+            CK(cudaEventRecord(d->pair_main, d->stream));
+            CK(cudaStreamWaitEvent(es, d->pair_main, 0));
+        }
         hook(swals::CAT_LINEAR_EDGE, 0);
-        CK(swals::launch_linear_pair_edge<R>(a, d->cfg, d->sc, d->aux.stream));
+        CK(swals::launch_linear_pair_edge<R>(a, d->cfg, d->sc, es));
         hook(swals::CAT_LINEAR_EDGE, 1);
-        CK(cudaEventRecord(d->pair_edge[k & 1], d->aux.stream));
+        if (beside) CK(cudaEventRecord(d->pair_edge[k & 1], es));
         d->cur = (d->cur + 1) % 3;
         d->nsteps += 2;
     }
-    if (npairs > 0) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[(npairs - 1) & 1], 0));
+    if (beside && npairs > 0) CK(cudaStreamWaitEvent(d->stream, d->pair_edge[(npairs - 1) & 1], 0));
     return SWALS_OK;
 }
 
@@ -838,7 +842,8 @@ extern "C" {
 // of the three state buffers, by one step or by a pair of linear steps, returns
 // to where it started; a graph reads and writes the buffers it was captured
 // with, so each starting buffer has its own.  Pairs take graphs of 24 steps
-// where they fit.  Timed (timers on) and first steps run one by one.
+// where they fit.  The first step and timed ones (timers on) are launched one
+// by one, timed linear steps still by pairs.
 static constexpr int GRAPH_STEPS[2] = {6, 24};
 
 static int step_graph(swals_domain *d, int which, double timestep, int32_t has_timestep, bool pairs)
