@@ -80,10 +80,8 @@ __device__ __forceinline__ R mc_double_gradient_ref(R local, R lower, R upper, R
 {
     const R a = upper - local;
     const R b = local - lower;
-    // (a NaN counts as negative, the sign that invalid operations give it:
-    // in a run that has blown up the sign decides how far it spreads)
-    const R sa = (a != a) ? R(-1) : copysign(R(1), a);
-    const R sb = (b != b) ? R(-1) : copysign(R(1), b);
+    const R sa = copysign(R(1), a);
+    const R sb = copysign(R(1), b);
     const R half_sasb = R(0.5) * (sa + sb);
     const R d = rmin(R(fabs(a)), R(fabs(b))) * half_sasb * th;
     const R e = R(0.5) * (a + b);
@@ -93,16 +91,17 @@ __device__ __forceinline__ R mc_double_gradient_ref(R local, R lower, R upper, R
 
 // The same for an ordinary theta (th2 is twice it): zero for different
 // signs, else min(|a + b|, min(|a|,|b|) 2 theta) with the sign of a; half the
-// instructions.
+// instructions.  Infinities and NaNs come out as they do there, a NaN's sign
+// included, by which the next step's sign products spread it.
 template <typename R>
 __device__ __forceinline__ R mc_double_gradient(R local, R lower, R upper, R th2)
 {
     const R a = upper - local;
     const R b = local - lower;
-    const R fa = R(fabs(a)), fb = R(fabs(b)), fe = R(fabs(a + b));
+    const R fa = R(fabs(a)), fb = R(fabs(b)), e = a + b, fe = R(fabs(e));
     const R d = rmin(fa, fb) * (same_sign(a, b) ? th2 : R(0));
     // (d zero is the answer whatever fe, which a NaN neighbour makes NaN)
-    return copysign((d < fe || bits_zero(d)) ? d : fe, a);
+    return (d < fe || bits_zero(d)) ? copysign(d, a) : e;
 }
 
 // theta_wd of DE1_inner_include.f90:751-757 / :813-819.
