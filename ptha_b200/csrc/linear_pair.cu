@@ -516,8 +516,6 @@ cudaError_t launch_pair(const LinearPair<R> &a, cudaStream_t s)
     const size_t smem =
         16 * 32 * (NLF ? 7 : 5) * SLOTS + sizeof(RowConst<R>) * (sh + 4) + (a.g_n > 0 ? 4 * (sh + 5) : 0);
     auto go = [&](auto kernel) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        if (e != cudaSuccess) return e;
         return launch_behind(kernel, (unsigned)ctas, 32, smem, s, a, sh, nstrips);
     };
     if (a.g_n > 0) return go(linear_pair_kernel<R, COR, TL, NLF, true>);
