@@ -110,9 +110,10 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
         c.dtj = COR ? dt * a.m.cor_be[r + 1] * half : zero;
         rc[k] = c;
     }
-    const pair::GaugeRows gauges(reinterpret_cast<int *>(rc + (SH + 4)), a.g_sites, GAUGES ? a.g_n : 0, ny, ra - 2,
-                                 rb - ra + 4, lane);
+    pair::GaugeRows gauges(reinterpret_cast<int *>(rc + (SH + 4)), a.g_sites, GAUGES ? a.g_n : 0, ny, ra - 2, rb - ra + 4,
+                           lane);
     __syncthreads();
+    if (GAUGES) gauges.ready(rb - ra + 4, lane);
     after_previous();   // (the metrics and gauge sites above are no kernel's output)
     let_next_start();
     const int rec = GAUGES ? (a.g_count ? *a.g_count : 0) : 0;
