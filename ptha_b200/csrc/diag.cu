@@ -14,8 +14,13 @@ __global__ void rounded_kernel(int op, const double *a, const double *b, int64_t
 {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
-    out[k] = op == SWALS_ROUNDED_RECIPROCAL ? rcp_ord(a[k]) : op == SWALS_ROUNDED_QUOTIENT ? div_ord(a[k], b[k])
-                                                                                           : sqrt_ord(a[k]);
+    switch (op) {
+    case SWALS_ROUNDED_RECIPROCAL: out[k] = rcp_ord(a[k]); break;
+    case SWALS_ROUNDED_QUOTIENT: out[k] = div_ord(a[k], b[k]); break;
+    case SWALS_ROUNDED_ROOT: out[k] = sqrt_ord(a[k]); break;
+    case SWALS_ROUNDED_RECIPROCAL_F32: out[k] = rcp_ord((float)a[k]); break;
+    default: out[k] = sqrt_ord((float)a[k]); break;
+    }
 }
 
 template <typename R>
@@ -242,7 +247,7 @@ template cudaError_t launch_timestep_max<float>(int, int, int64_t, const float *
 
 extern "C" int swals_gpu_rounded(int32_t op, const double *a, const double *b, int64_t n, double *out)
 {
-    if (op < SWALS_ROUNDED_RECIPROCAL || op > SWALS_ROUNDED_ROOT || !a || !out || n < 1 || n > (int64_t(1) << 30) ||
+    if (op < SWALS_ROUNDED_RECIPROCAL || op > SWALS_ROUNDED_ROOT_F32 || !a || !out || n < 1 || n > (int64_t(1) << 30) ||
         (op == SWALS_ROUNDED_QUOTIENT && !b))
         return swals::api_fail(SWALS_ERR_INVALID_ARGUMENT, "bad argument");
     if (op != SWALS_ROUNDED_QUOTIENT) b = nullptr;

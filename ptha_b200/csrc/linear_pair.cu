@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
                         vv = vv - k.cv[c] * u4;
                     }
                     if (NLF) {
-                        uu = friction_multiplier(one + a.lin_fric_dt, dt, fu[c], u[c], half * v4) * uu;
-                        vv = friction_multiplier(one + a.lin_fric_dt, dt, fv[c], v[c], half * u4) * vv;
+                        uu = friction_multiplier_line(one + a.lin_fric_dt, dt, fu[c], u[c], half * v4) * uu;
+                        vv = friction_multiplier_line(one + a.lin_fric_dt, dt, fv[c], v[c], half * u4) * vv;
                     }
                 }
                 if (!NLF && a.lin_fric) {

@@ -438,9 +438,11 @@ __device__ __forceinline__ R friction_factor(const Rk2Args<R> &a, R nsq, const C
     const R depth = c.dep;
     const R speed2 = c.u * c.u + c.v * c.v;
     const R dg = dt * K<R>::gravity() * rmax(depth, R(0));
-    if ((double)depth < 1.0e30 && (double)speed2 < 1.0e280) {
+    const R large = sizeof(R) == 8 ? R(1.0e280) : R(1.0e37);
+    if ((double)depth < 1.0e30 && speed2 < large) {
         const R fs = nsq * sqrt_ord(speed2) * R(pow_friction<CHEZY, true>((double)rmax(depth, mad)));
-        return rcp_ord((R(1) + dg * fs) + dt * a.lin_fric);
+        const R d = (R(1) + dg * fs) + dt * a.lin_fric;
+        if (sizeof(R) == 8 || d < large) return rcp_ord(d);
     }
     // a run that has blown up: the plain operators
     const R fs = nsq * R(sqrt(speed2)) * R(pow_friction<CHEZY>((double)rmax(depth, mad)));

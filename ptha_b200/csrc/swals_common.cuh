@@ -77,7 +77,6 @@ __device__ __forceinline__ double rcp_ord(double b)
 {
     return rcp_of_ones(b, rcp_step(b, rcp_step(b, rcp_step(b, rcp_seed(b)))));
 }
-__device__ __forceinline__ float rcp_ord(float b) { return 1.0f / b; }
 __device__ __forceinline__ double div_ord(double a, double b)
 {
     const double y1 = rcp_step(b, rcp_seed(b));
@@ -100,7 +99,36 @@ __device__ __forceinline__ double sqrt_ord(double x)
     g = fma(fma(-g, g, x), h, g);
     return (x < 1.0e-290) ? 0.0 : g;
 }
-__device__ __forceinline__ float sqrt_ord(float x) { return sqrtf(x); }
+// The same in FP32, for roots up to 2^126 and reciprocals of 2^-125 .. 2^125:
+// the general operators branch on zeros and subnormals, and a few such lanes
+// hold up their warp.  Friction pairs, us a step, general with waves everywhere
+// / general with half the grid at rest / these: 500 x 700 13.2 / 18.9 / 9.9
+// (single steps 13.1), 2000 x 1500 35.1 / 48.4 / 28.0.
+// Below 2^-80, where the squares of fading momenta end (subnormals and zero
+// included), a root is that of x 2^96 times 2^-48: exact, but that zero gives
+// 2^-111, which is lost beside the 1 that the friction terms add to.
+__device__ __forceinline__ float rcp_ord(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    y = fma(y, fma(-b, y, 1.0f), y);
+    y = fma(y, fma(-b, y, 1.0f), y);
+    const int i = __float_as_int(b);
+    return __int_as_float(__float_as_int(y) | ((i & 0x7fffff) == 0x7fffff ? 1 : 0));
+}
+__device__ __forceinline__ float sqrt_ord(float x)
+{
+    const bool small = x < 0x1p-80f;
+    const float s = small ? fma(x, 0x1p96f, 0x1p-126f) : x;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    float g = s * y, h = 0.5f * y;
+    const float r = fma(-g, h, 0.5f);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    g = fma(fma(-g, g, s), h, g);
+    return small ? g * 0x1p-48f : g;
+}
 
 // 1 / depth of a wet cell.
 __device__ __forceinline__ double depth_inverse(double dep) { return dep < 1.0e280 ? rcp_ord(dep) : 1.0 / dep; }
@@ -117,6 +145,20 @@ __device__ __forceinline__ double friction_multiplier(double lf1, double dt, dou
 __device__ __forceinline__ float friction_multiplier(float lf1, float dt, float fw, float m0, float mt)
 {
     return 1.0f / (lf1 + dt * fw * sqrtf(m0 * m0 + mt * mt));
+}
+// For kernels whose few warps do not fill the branches of the general FP32
+// operators (where many do, those are faster: leapfrog_nonlinear 2000 x 1500
+// 152 us a step, by these 155).
+__device__ __forceinline__ double friction_multiplier_line(double lf1, double dt, double fw, double m0, double mt)
+{
+    return friction_multiplier(lf1, dt, fw, m0, mt);
+}
+__device__ __forceinline__ float friction_multiplier_line(float lf1, float dt, float fw, float m0, float mt)
+{
+    const float x = m0 * m0 + mt * mt;
+    const float d = lf1 + dt * fw * sqrt_ord(x);
+    if (x < 1.0e37f && d < 1.0e37f) return rcp_ord(d);
+    return 1.0f / (lf1 + dt * fw * sqrtf(x));   // a run that has blown up
 }
 
 // Friction power law pow(x, p), p = fl(-7/3) (Manning) or -2 (Chezy), for
