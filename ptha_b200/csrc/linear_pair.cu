@@ -338,7 +338,6 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
             east(e1, ee);
             faces(k1, e1, ee, e, a1, ae, sA, k1f);
             momenta(r - 1, k1.dxb1, u1, v1, a1, ae, sA, k1f, hv2, hu1, hu, f1, g1, uA, vA, hv);
-            if (GAUGES && r - 1 >= ra && r - 1 < rb) record(0, r - 1, a1, uA, vA);
             if (a.lines && r - 1 >= ra && r - 1 < rb) {
                 const int j = r - 1;
                 if (out && (j == ny - a.n_ext - 1 || j == a.n_ext - 1)) {
@@ -408,7 +407,11 @@ __global__ void __launch_bounds__(32, pair_warps(NLF, (int)sizeof(R))) linear_pa
                         }
                 }
             }
-            if (GAUGES && q >= ra) record(1, q, b2, uB, vB);
+            // gauges: step 1 on row r-1, step 2 on row r-2
+            if (GAUGES && (gauges.on(r - 1 - (ra - 2)) || gauges.on(q - (ra - 2)))) {
+                if (r - 1 >= ra && r - 1 < rb) record(0, r - 1, a1, uA, vA);
+                if (q >= ra) record(1, q, b2, uB, vB);
+            }
 #pragma unroll
             for (int c = 0; c < CPL; c++) {
                 e2[c] = e1[c];
