@@ -483,9 +483,10 @@ int swals_gpu_volume_in_priority_domain(swals_domain *d, double *out);
 
 /* The library's straight-line FP64 reciprocal 1/a, quotient a/b and square
  * root of a on host arrays of n values: correctly rounded for operands and
- * results between 1e-290 and 1e290 (roots of less, zero included, are zero);
- * the FP32 ones of (float)a: reciprocals of 2^-125 .. 2^125, roots up to 2^126
- * (of zero 2^-111). */
+ * results between 1e-290 and 1e290 (roots of less, zero included, are zero, of
+ * more they are right up to the largest number, of infinity NaN); the FP32 ones
+ * of (float)a: reciprocals of 2^-125 .. 2^125, all finite roots (of zero
+ * 2^-111). */
 enum {
     SWALS_ROUNDED_RECIPROCAL = 0, SWALS_ROUNDED_QUOTIENT = 1, SWALS_ROUNDED_ROOT = 2,
     SWALS_ROUNDED_RECIPROCAL_F32 = 3, SWALS_ROUNDED_ROOT_F32 = 4

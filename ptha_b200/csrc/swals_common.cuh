@@ -56,7 +56,7 @@ template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return (b > 
 // The callers see to the range and use the plain operators outside it:
 // operands, results and remainders between 1e-290 and 1e290, so that nothing
 // overflows, underflows or is infinite.  sqrt_ord takes what is below 1e-290,
-// zero included, as zero.
+// zero included, as zero, anything finite above, and gives NaN for infinity.
 // A step of Newton's iteration for 1/b.
 __device__ __forceinline__ double rcp_step(double b, double y) { return fma(y, fma(-b, y, 1.0), y); }
 __device__ __forceinline__ double rcp_seed(double b)
@@ -99,11 +99,11 @@ __device__ __forceinline__ double sqrt_ord(double x)
     g = fma(fma(-g, g, x), h, g);
     return (x < 1.0e-290) ? 0.0 : g;
 }
-// The same in FP32, for roots up to 2^126 and reciprocals of 2^-125 .. 2^125:
+// The same in FP32, for reciprocals of 2^-125 .. 2^125 and all finite roots:
 // the general operators branch on zeros and subnormals, and a few such lanes
 // hold up their warp.  Friction pairs, us a step, general with waves everywhere
-// / general with half the grid at rest / these: 500 x 700 13.2 / 18.9 / 9.9
-// (single steps 13.1), 2000 x 1500 35.1 / 48.4 / 28.0.
+// / general with half the grid at rest / these: 500 x 700 13.2 / 18.9 / 9.4
+// (single steps 13.1), 2000 x 1500 35.1 / 48.4 / 26.8.
 // Below 2^-80, where the squares of fading momenta end (subnormals and zero
 // included), a root is that of x 2^96 times 2^-48: exact, but that zero gives
 // 2^-111, which is lost beside the 1 that the friction terms add to.
@@ -146,19 +146,27 @@ __device__ __forceinline__ float friction_multiplier(float lf1, float dt, float 
 {
     return 1.0f / (lf1 + dt * fw * sqrtf(m0 * m0 + mt * mt));
 }
-// For kernels whose few warps do not fill the branches of the general FP32
-// operators (where many do, those are faster: leapfrog_nonlinear 2000 x 1500
-// 152 us a step, by these 155).
+// For kernels whose few warps do not fill one another's branches: formed first
+// and replaced where it must be, so that the next face's goes beside it.
+// Friction pairs 1501 x 1001 FP64, the branch first / this: with Coriolis 28.5 /
+// 28.2 us a step, without 28.1 / 27.2; leapfrog_nonlinear, whose warps are many,
+// is faster by the branch (1024 x 768 FP64 54.1 / 54.5, 2000 x 1500 FP32 152 /
+// 155).
 __device__ __forceinline__ double friction_multiplier_line(double lf1, double dt, double fw, double m0, double mt)
 {
-    return friction_multiplier(lf1, dt, fw, m0, mt);
+    const double x = m0 * m0 + mt * mt;
+    const double d = lf1 + dt * fw * sqrt_ord(x);
+    double r = rcp_ord(d);
+    if (!(d < 1.0e280)) r = 1.0 / (lf1 + dt * fw * sqrt(x));   // a run that has blown up
+    return r;
 }
 __device__ __forceinline__ float friction_multiplier_line(float lf1, float dt, float fw, float m0, float mt)
 {
     const float x = m0 * m0 + mt * mt;
     const float d = lf1 + dt * fw * sqrt_ord(x);
-    if (x < 1.0e37f && d < 1.0e37f) return rcp_ord(d);
-    return 1.0f / (lf1 + dt * fw * sqrtf(x));   // a run that has blown up
+    float r = rcp_ord(d);
+    if (!(d < 1.0e37f)) r = 1.0f / (lf1 + dt * fw * sqrtf(x));   // a run that has blown up
+    return r;
 }
 
 // Friction power law pow(x, p), p = fl(-7/3) (Manning) or -2 (Chezy), for

@@ -50,8 +50,9 @@ def test_random_operands():
     _same(_rounded(RECIPROCAL, b), 1.0 / b)
     a, b = _operands(rng, N, -481, 480) * rng.choice([-1.0, 1.0], N), _operands(rng, N, -481, 480)
     _same(_rounded(QUOTIENT, a, b), a / b)
-    x = _operands(rng, N, -963, 962)
+    x = _operands(rng, N, -963, 1023)
     _same(_rounded(ROOT, x), np.sqrt(x))
+    assert np.isnan(_rounded(ROOT, np.array([np.inf, np.nan]))).all()
 
 
 def test_ends_of_the_range():
@@ -130,6 +131,6 @@ def test_roots_next_to_a_middle():
     assert len(X) > 250
     x = np.array(X, dtype=np.int64).astype(np.float64)
     assert all(int(v) == q for v, q in zip(x, X))
-    for e in (-52, -1012, -512, 0, 500, 900):
+    for e in (-52, -1012, -512, 0, 500, 900, 970):
         y = np.ldexp(x, e)
         _same(_rounded(ROOT, y), np.sqrt(y))
