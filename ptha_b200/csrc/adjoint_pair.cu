@@ -17,9 +17,10 @@
 //
 // A pass moves 56 B a cell (FP64) for two steps.  The single-step kernel is
 // held by its 8-byte loads, shuffles and selects, not by memory.  Measured on
-// the B200, us a step, that kernel / this one: 1200 x 800 FP64 Coriolis 23.0 /
-// 12.0 (rows per segment 6 12.8, 10 12.3, 16 13.8), 3600 x 2400 145 / 57 (4.2
-// TB/s), 1800 x 1200 FP32 33.5 / 14.9, 400^2 FP64 with 9 gauges 12.4 / 5.2.
+// the B200, us a step, that kernel / this one: 1200 x 800 FP64 Coriolis 22.8 /
+// 10.1 (rows per segment one after another 6 12.8, 10 12.3, 16 13.8), 3600 x
+// 2400 146 / 58 (4.2 TB/s), 1800 x 1200 FP32 32.8 / 12.9, 400^2 FP64 with 9
+// gauges 12.3 / 4.0.
 #include <type_traits>
 
 #include "pair_common.cuh"
@@ -32,7 +33,7 @@ using pair::cp16;
 
 constexpr int SLOTS = 4;    // ring slots: row r, two in flight, and row r-1's ELV
 constexpr int NP = 4;       // lambda_STG, lambda_UH, lambda_VH of row r, ELV of row r+1
-constexpr int RESIDENT = 12;  // warps per SM (154 registers a thread)
+constexpr int RESIDENT = 12;  // warps per SM (160 registers a thread)
 
 template <typename R> __device__ __forceinline__ void cp_one(R *smem, const R *gmem, bool in)
 {

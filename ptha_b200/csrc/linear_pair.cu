@@ -24,7 +24,7 @@
 // of a wet face (truly linear solver) both steps, the row constants (dt / area
 // and so on) the whole strip; a segment away from the sides selects nothing.
 // 112 -> 93 thread instructions a cell and step, 3600 x 2400 FP32
-// Coriolis 43.7 -> 36.8 us a step.  Products and sums keep the single step's
+// Coriolis 43.7 -> 36.3 us a step.  Products and sums keep the single step's
 // operands and order, so the results are the same bits.
 //
 // 16-byte lanes start on 16-byte boundaries (strips every 480 bytes, 15 whole
@@ -32,11 +32,11 @@
 // lanes with twice the warps are no faster (FP32 38.3).
 //
 // Measured on the B200, us a step, one step at a time / in pairs: 4096^2 FP64
-// 212 / 112, 8192^2 791 / 421 (a pair moves 72 B a cell: 5.4 and 5.7 TB/s,
-// 0.84 and 0.89 of the copy bandwidth), FP32 111 / 60, 3600 x 2400 FP32
-// Coriolis 71.3 / 36.8, 1200 x 800 Coriolis 20.5 / 11.0, 400^2 with 9 gauges
-// 9.3 / 5.4, 200 x 150 7.6 / 3.5; with Manning friction 1501 x 1001 Coriolis
-// 58.6 / 29.0, 3000 x 2000 FP32 120 / 64.
+// 212 / 113, 8192^2 787 / 427 (a pair moves 72 B a cell: 5.3 and 5.7 TB/s,
+// 0.83 and 0.88 of the copy bandwidth), FP32 111 / 62, 3600 x 2400 FP32
+// Coriolis 71.6 / 36.3, 1200 x 800 Coriolis 20.5 / 10.5, 400^2 with 9 gauges
+// 9.4 / 4.9, 200 x 150 7.2 / 3.3; with Manning friction 1501 x 1001 Coriolis
+// 58.0 / 28.2, 3000 x 2000 FP32 114 / 45.7.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

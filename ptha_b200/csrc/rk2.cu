@@ -603,7 +603,7 @@ cudaError_t launch_stage_stream(const fv::Rk2Args<R> &a, cudaStream_t s);
 
 namespace {
 
-// Stage kernel variant: register streaming (default) or shared-memory tiles,
+// Stage kernel variant: CTA-wide strips (default) or shared-memory tiles,
 // chosen by SWALS_FV_KERNEL=stream|tile.
 bool use_stream_kernel()
 {

@@ -1,5 +1,5 @@
 // rk2_common.cuh -- device pieces shared by the finite-volume stage kernels
-// (rk2.cu: shared-memory tiles; rk2_stream.cu: register streaming).
+// (rk2.cu: shared-memory tiles; rk2_stream.cu: CTA-wide strips).
 #pragma once
 #include "swals_kernels.h"
 

@@ -14,9 +14,9 @@
 //   - the next row's loads are issued before the current row is processed,
 //     the lines that only the update reads are started towards L2, and stage 2
 //     loads them a barrier ahead.
-// Bound by instruction issue: 2048^2 FP64 stage 2 254 us, 1480 thread
+// Bound by instruction issue: 2048^2 FP64 stage 2 250 us, 1455 thread
 // instructions a cell, 72 % of the issue slots, FP64 pipe 49 % busy; the flux
-// pass 207 us, 1121, 68 %, 49 % (1792 and 1523 instructions, 315 and 263 us,
+// pass 205 us, 1095, 68 %, 50 % (1792 and 1523 instructions, 315 and 263 us,
 // before the straight-line roots and quotients and the sign-free limiter).
 #include "rk2_common.cuh"
 

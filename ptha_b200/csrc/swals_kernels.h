@@ -152,9 +152,10 @@ cudaError_t launch_domain_statistics(int nx, int ny, int64_t P, const R *stg, co
                                      double *rows6, double *out7, cudaStream_t s);
 
 // Gauges (0-based i, j site pairs) inside the window [i0, i1] x [r0, r1]:
-// bit q set for gauge q.  Streaming kernels compute it once per warp segment
-// so the per-row check costs nothing where there is no gauge.  With more than
-// 64 gauges every bit is set and the callers test each gauge.
+// bit q set for gauge q.  The streaming kernels of single steps compute it once
+// per warp segment so the per-row check costs nothing where there is no gauge;
+// with more than 64 gauges every bit is set and they test each gauge.  (The
+// two-steps-a-pass kernels go by the index below instead.)
 __device__ __forceinline__ unsigned long long gauges_in(const int *sites, int n, int i0, int i1, int r0, int r1)
 {
     if (n > 64) return ~0ull;
