@@ -132,3 +132,22 @@ def test_series_ending_within_a_pair(capacity):
             out.append(rec)
     assert np.abs(out[0][-1]).max() > 0.0
     np.testing.assert_array_equal(out[0], out[1])
+
+
+def test_failed_setup_leaves_no_sites():
+    """A gauge outside the domain is refused, and nothing is left of the others."""
+    kw, U = _case(8)
+    with Domain(**kw) as d:
+        d.set_U(U)
+        dt = 0.5 * d.linear_timestep_max()
+        xy = _xy(kw, _cells("twice"))
+        d.gauges_setup(xy, 20)
+        with pytest.raises(_lib.SwalsError, match="outside the domain"):
+            d.gauges_setup(np.concatenate([xy[:3], [[1.0e9, -1.0e9]]]), 20)
+        with pytest.raises(_lib.SwalsError, match="gauges must be set up first"):
+            d.misfit_gradient(4, dt, np.zeros((4, 4)), checkpoint_every=2)
+        d.evolve_steps(6, dt)
+        assert np.isfinite(d.get_U()).all()
+        d.gauges_setup(xy, 20)
+        d.evolve_steps(6, dt)
+        assert d.gauges_read().shape == (6, len(xy), 3)
